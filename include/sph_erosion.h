@@ -118,19 +118,22 @@ typedef struct sph_system_config {
                                      neighbours (192 slots, 772 B per particle) and the
                                      force pass reads them instead of re-testing the
                                      cells; ignored when the HBM budget has no room,
-                                16 = with 8: the force pass's list walk loads ahead,
+                                16 = with 8: the force pass's list walk loads ahead (every
+                                     list walk does now; fast arithmetic still asks for it),
                                 32 = with 8: relaxed register budget of the density pass only,
                                 64 = with 8: the density pass loads candidates in pairs,
                                128 = with 8: the force pass gathers one packed 32-byte
-                                     record per neighbour (32 more bytes per particle),
+                                     record per neighbour (32 more bytes per particle,
+                                     part of the variant's memory; without the bit they
+                                     are used too while the HBM budget has room),
                                256 = with 8: cooperative passes, a group of lanes per
                                      particle: the density pass sweeps the particle's
                                      candidates 32 at a time (2048: 16 lanes), the force
                                      pass splits its list over 8 lanes (512: 4, 1024: 16);
                                      with 256, bit 4 relaxes the force pass's registers,
                              32768 = with 8 + 16: the force pass's warps take their work
-                                     in 32-particle slices from a counter instead of one
-                                     block per tile (65536: the density pass's); same bits,
+                                     in 32-particle slices from a counter (they always do
+                                     now; 65536: the density pass's); same bits,
                             131072 = with 8 + 16: fast arithmetic in both neighbour passes
                                      (grouped products, fused multiply-adds, r^2 for
                                      |r|^2, hardware 1/sqrt); exact in-range test, so the

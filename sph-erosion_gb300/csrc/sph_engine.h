@@ -155,7 +155,7 @@ class System {
     void capture_graph();
     void advance_step_mirror(int nsteps);
     void drop_graph();
-    void check_budget(int64_t extra) const;
+    void check_budget(int64_t extra);
     void upload_terrain_height(Scene& sc);
 
     sph_system_config cfg_;

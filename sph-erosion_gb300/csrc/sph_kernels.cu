@@ -55,13 +55,45 @@ __device__ __forceinline__ float dist2(float dx, float dy, float dz) {
     return fa(fa(fm(dx, dx), fm(dy, dy)), fm(dz, dz));
 }
 
-// Two consecutive float4 (32 bytes at a 32-byte boundary: a packed record,
-// or two neighbouring sorted positions) in one 256-bit read-only load, one
-// L1 request instead of two.
-__device__ __forceinline__ void ld_record(const float4* p, float4& a, float4& b) {
-    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-        : "l"(p));
+// Two floats in one 64-bit register pair and the packed FP32 operations on
+// them (sm_100 and later): one instruction for two operations, each half
+// rounded like its scalar form, so they change no bits.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pk(float lo, float hi) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ f2 pk(float v) { return pk(v, v); }
+__device__ __forceinline__ float lo(f2 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float hi(f2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) { return fma2(a, pk(1.0f), b); }
+// A product that an addition follows, as a * b + (-0) with the -0 read from
+// memory: the assembler fuses mul.rn.f32x2 into an addition that uses its
+// result (also into a scalar one), which would drop the product's rounding;
+// this form it cannot fuse.
+__constant__ float kNegZero[2] = {-0.0f, -0.0f};
+__device__ __forceinline__ f2 mulr2(f2 a, f2 b) { return fma2(a, b, pk(kNegZero[0], kNegZero[1])); }
+
+// A packed neighbour record (DevArrays::fdat) as four pairs: (x, y),
+// (z, P/rho^2), (vx, vy), (vz, m/rho); one 256-bit load.
+struct Rec {
+    f2 xy, zA, vxy, vzB;
+};
+__device__ __forceinline__ Rec ld_rec(const float4* p) {
+    Rec r;
+    asm("ld.global.nc.v4.b64 {%0,%1,%2,%3}, [%4];" : "=l"(r.xy), "=l"(r.zA), "=l"(r.vxy), "=l"(r.vzB) : "l"(p));
+    return r;
 }
 
 __device__ __forceinline__ int cell_coord(float x, float lo, float inv, int n) {
@@ -938,11 +970,11 @@ __device__ __forceinline__ void integrate_and_store(const DevArrays& a, const Sc
 // force: passes 2 and 3 (fluid_system.h:127-178) and advance (:306-353) with
 // the terrain contact, the box collision and the erosion exchange.
 // NL: the in-range neighbours come from the lists the density pass wrote
-// (same order as the traversal, so the same sums); a particle whose list
-// overflowed walks its cells instead.  NL = 2
-// software-pipelines the list walk: list entries two ahead and the
-// neighbour's state one ahead are loaded before the current pair is summed.
-template <bool ORDERED, int MINB, int NL = 0, bool DYN = false, bool FM = false>
+// (same order as the traversal, so the same sums), list entries two ahead and
+// the neighbour's state one ahead; a particle whose list overflowed walks its
+// cells instead.  This form gathers from the three sorted arrays: it serves
+// systems whose HBM budget has no room for the packed records (k_force_rec).
+template <bool ORDERED, int MINB, bool NL = false, bool DYN = false, bool FM = false>
 __global__ void __launch_bounds__(kMaxTile, MINB) k_force(DevArrays a) {
     extern __shared__ uint32_t list[];
     const int nwork = *a.n_ptiles;
@@ -991,13 +1023,7 @@ __global__ void __launch_bounds__(kMaxTile, MINB) k_force(DevArrays a) {
                 for_each_candidate(a, S, xi, [&](uint32_t j, float4 xj) {
                     if (dist2(fs(xi.x, xj.x), fs(xi.y, xj.y), fs(xi.z, xj.z)) <= S.smax) pair(j, xj);
                 });
-            } else if (NL == 1) {
-                const uint32_t* nl = a.nlist + (size_t)wk.start * kNbCap + li;
-                for (int q = 0; q < cnt; ++q) {
-                    const uint32_t j = __ldg(nl + (size_t)q * lstride);
-                    pair(j, __ldg(sp + j));
-                }
-            } else if (NL == 2) {
+            } else {
                 const uint32_t* nl = a.nlist + (size_t)wk.start * kNbCap + li;
                 const int stride = lstride;
                 uint32_t j0 = cnt > 0 ? __ldg(nl) : 0u;
@@ -1024,39 +1050,250 @@ __global__ void __launch_bounds__(kMaxTile, MINB) k_force(DevArrays a) {
                     v0 = v1;
                     d0 = d1;
                 }
-            } else {
-                // NL == 3: the same walk over the packed 32-byte records (one
-                // sector per neighbour); the id is read only in record mode
-                const uint32_t* nl = a.nlist + (size_t)wk.start * kNbCap + li;
-                const int stride = lstride;
-                const float4* fd = a.fdat + 2 * (size_t)S.p_off;
-                const bool rec = (S.flags & kFlagRecord) != 0;
-                uint32_t j0 = cnt > 0 ? __ldg(nl) : 0u;
-                uint32_t j1 = cnt > 1 ? __ldg(nl + stride) : 0u;
-                float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), b0 = a0;
-                if (cnt > 0) ld_record(fd + 2 * j0, a0, b0);
-                nl += 2 * stride;
-                for (int q = 0; q < cnt; ++q, nl += stride) {
-                    const uint32_t j2 = (q + 2 < cnt) ? __ldg(nl) : 0u;
-                    float4 a1 = a0, b1 = b0;
-                    if (q + 1 < cnt) ld_record(fd + 2 * j1, a1, b1);
-                    const int idj = rec ? __float_as_int(__ldg(&sp[j0].w)) : 0;
-                    const float rx = fs(xi.x, a0.x), ry = fs(xi.y, a0.y), rz = fs(xi.z, a0.z);
-                    if (FM)
-                        force_pair_fast(S, acc, rx, ry, rz, dist2_fma(rx, ry, rz), vi.x, vi.y, vi.z, Ai, b0, a0.w, b0.w,
-                                        idj, (int)j0 == pl);
-                    else
-                        force_pair(S, acc, rx, ry, rz, fsq(dist2(rx, ry, rz)), vi.x, vi.y, vi.z, Ai, b0, a0.w, b0.w,
-                                   idj, (int)j0 == pl);
-                    j0 = j1;
-                    j1 = j2;
-                    a0 = a1;
-                    b0 = b1;
-                }
             }
             if (!valid) continue;
         }
         integrate_and_store(a, S, p, xi, vi, rho, acc, true);
+    }
+}
+
+// Sum of the pair terms of two list neighbours A and B (A first), the terms
+// of both computed together in packed operations; each term and each sum
+// rounds as in force_pair (FM: force_pair_fast).  nr = x_j - x_i is the
+// negative of the reference's r and every coefficient that multiplies it is
+// negated, which changes no bits.  The particle itself (s = 0) needs no test:
+// its r and its velocity difference are zero, so it adds zeros to all sums but
+// the colour field's, where it belongs; only the reciprocal length is kept
+// finite.  Coincident neighbours (s below the threshold) must not come here.
+struct PairIn {
+    float x, y, z;     // x_j - x_i
+    float vx, vy, vz;  // v_j - v_i
+    float AA, B;       // A_i + A_j, m/rho_j
+    float s;           // |x_j - x_i|^2
+};
+
+struct PairConst {
+    float h, hh, hh3, cg, cs, mass, clamp;
+};
+
+template <bool FM>
+__device__ __forceinline__ void force_two(const PairConst& K, ForceAcc& acc, const PairIn& a, const PairIn& b,
+                                          float lapB) {
+    const f2 S2 = pk(a.s, b.s);
+    if (FM) {
+        const f2 hs = fma2(S2, pk(-1.0f), pk(K.hh));
+        const f2 lap = mul2(mul2(hs, pk(K.cg)), fma2(S2, pk(-7.0f), pk(K.hh3)));
+        acc.cfl = fmaf(-a.B, lo(lap), acc.cfl);
+        acc.cfl = fmaf(-lapB, hi(lap), acc.cfl);
+        const f2 inv = pk(rsqrtf(fmaxf(a.s, K.clamp)), rsqrtf(fmaxf(b.s, K.clamp)));
+        const f2 w = fma2(S2, inv, pk(-K.h));  // |r| - h
+        const f2 coef = mul2(pk(a.AA, b.AA), pk(K.mass));
+        const f2 g = mul2(mul2(mul2(coef, pk(K.cs)), mul2(w, w)), inv);
+        const f2 lv = mul2(w, pk(K.cs));
+        const f2 gn = mul2(mul2(pk(a.B, b.B), pk(K.cg)), mul2(hs, hs));
+        const f2 bl = mul2(pk(a.B, b.B), lv);
+        acc.fpx = fmaf(a.x, lo(g), acc.fpx);
+        acc.fpy = fmaf(a.y, lo(g), acc.fpy);
+        acc.fpz = fmaf(a.z, lo(g), acc.fpz);
+        acc.fvx = fmaf(a.vx, -lo(bl), acc.fvx);
+        acc.fvy = fmaf(a.vy, -lo(bl), acc.fvy);
+        acc.fvz = fmaf(a.vz, -lo(bl), acc.fvz);
+        acc.nx = fmaf(a.x, lo(gn), acc.nx);
+        acc.ny = fmaf(a.y, lo(gn), acc.ny);
+        acc.nz = fmaf(a.z, lo(gn), acc.nz);
+        acc.fpx = fmaf(b.x, hi(g), acc.fpx);
+        acc.fpy = fmaf(b.y, hi(g), acc.fpy);
+        acc.fpz = fmaf(b.z, hi(g), acc.fpz);
+        acc.fvx = fmaf(b.vx, -hi(bl), acc.fvx);
+        acc.fvy = fmaf(b.vy, -hi(bl), acc.fvy);
+        acc.fvz = fmaf(b.vz, -hi(bl), acc.fvz);
+        acc.nx = fmaf(b.x, hi(gn), acc.nx);
+        acc.ny = fmaf(b.y, hi(gn), acc.ny);
+        acc.nz = fmaf(b.z, hi(gn), acc.nz);
+    } else {
+        const float la = fsq(a.s), lb = fsq(b.s);
+        const f2 cg = pk(K.cg);
+        const f2 L = pk(la, lb);
+        const f2 hs = fma2(mulr2(L, L), pk(-1.0f), pk(K.hh));
+        const f2 lap = mul2(mul2(cg, hs), fma2(mulr2(mul2(pk(7.0f), L), L), pk(-1.0f), pk(K.hh3)));
+        const f2 lB = mulr2(pk(-a.B, -lapB), lap);
+        acc.cfl = fa(acc.cfl, lo(lB));
+        acc.cfl = fa(acc.cfl, hi(lB));
+        const f2 inv = pk(__frcp_rn(fmaxf(la, K.clamp)), __frcp_rn(fmaxf(lb, K.clamp)));
+        const f2 d = fma2(L, pk(-1.0f), pk(K.h));  // h - |r|
+        const f2 pw2 = mul2(d, d), cs = pk(K.cs);
+        const f2 coef = mul2(pk(a.AA, b.AA), pk(K.mass));
+        const f2 B = pk(a.B, b.B);
+        const f2 lv = mul2(cs, d);
+        const f2 pw = mul2(hs, hs);
+        const f2 x = pk(a.x, b.x), y = pk(a.y, b.y), z = pk(a.z, b.z);
+        const f2 gx = mulr2(coef, mul2(mul2(mul2(x, inv), cs), pw2));
+        const f2 gy = mulr2(coef, mul2(mul2(mul2(y, inv), cs), pw2));
+        const f2 gz = mulr2(coef, mul2(mul2(mul2(z, inv), cs), pw2));
+        acc.fpx = fa(fa(acc.fpx, lo(gx)), hi(gx));
+        acc.fpy = fa(fa(acc.fpy, lo(gy)), hi(gy));
+        acc.fpz = fa(fa(acc.fpz, lo(gz)), hi(gz));
+        const f2 vx = mulr2(mul2(pk(a.vx, b.vx), B), lv);
+        const f2 vy = mulr2(mul2(pk(a.vy, b.vy), B), lv);
+        const f2 vz = mulr2(mul2(pk(a.vz, b.vz), B), lv);
+        acc.fvx = fa(fa(acc.fvx, lo(vx)), hi(vx));
+        acc.fvy = fa(fa(acc.fvy, lo(vy)), hi(vy));
+        acc.fvz = fa(fa(acc.fvz, lo(vz)), hi(vz));
+        const f2 nx = mulr2(B, mul2(mul2(x, cg), pw));
+        const f2 ny = mulr2(B, mul2(mul2(y, cg), pw));
+        const f2 nz = mulr2(B, mul2(mul2(z, cg), pw));
+        acc.nx = fa(fa(acc.nx, lo(nx)), hi(nx));
+        acc.ny = fa(fa(acc.ny, lo(ny)), hi(ny));
+        acc.nz = fa(fa(acc.nz, lo(nz)), hi(nz));
+    }
+}
+
+template <bool FM>
+__device__ __forceinline__ PairIn pair_in(const Rec& r, float nxi, float nyi, float nzi, float Ai, float nvx, float nvy,
+                                          float nvz) {
+    PairIn q;
+    if (FM) {
+        const f2 xy = add2(r.xy, pk(nxi, nyi)), zA = add2(r.zA, pk(nzi, Ai)), vxy = add2(r.vxy, pk(nvx, nvy));
+        q.x = lo(xy), q.y = hi(xy), q.z = lo(zA), q.AA = hi(zA), q.vx = lo(vxy), q.vy = hi(vxy);
+    } else {
+        q.x = fa(lo(r.xy), nxi), q.y = fa(hi(r.xy), nyi), q.z = fa(lo(r.zA), nzi), q.AA = fa(hi(r.zA), Ai);
+        q.vx = fa(lo(r.vxy), nvx), q.vy = fa(hi(r.vxy), nvy);
+    }
+    q.vz = fa(lo(r.vzB), nvz);
+    q.B = hi(r.vzB);
+    q.s = FM ? dist2_fma(q.x, q.y, q.z) : dist2(q.x, q.y, q.z);
+    return q;
+}
+
+// One pair in the general form: the particle itself adds to the colour field
+// only, a coincident neighbour takes the fixed direction.
+template <bool FM>
+__device__ __forceinline__ void force_one(const SceneDev& S, ForceAcc& acc, const PairIn& q, bool self) {
+    const float4 dv = make_float4(q.vx, q.vy, q.vz, 0.0f);
+    if (FM)
+        force_pair_fast(S, acc, -q.x, -q.y, -q.z, q.s, 0.0f, 0.0f, 0.0f, q.AA, dv, 0.0f, q.B, -1, self);
+    else
+        force_pair(S, acc, -q.x, -q.y, -q.z, fsq(q.s), 0.0f, 0.0f, 0.0f, q.AA, dv, 0.0f, q.B, -1, self);
+}
+
+// The neighbour sums of a particle whose list overflowed: it walks its cells
+// (same order).  A call, so that this rare path takes no registers from the
+// list walk.
+template <bool FM>
+__device__ __noinline__ void force_cells(const DevArrays& a, const SceneDev& S, int p, ForceAcc& acc) {
+    const int pl = p - S.p_off;
+    const float4 xi = a.spos[p], vi = a.svel[p], di = a.dyn[p];
+    const float4* sv = a.svel + S.p_off;
+    const float4* sd = a.dyn + S.p_off;
+    for_each_candidate(a, S, xi, [&](uint32_t j, float4 xj) {
+        const float rx = fs(xi.x, xj.x), ry = fs(xi.y, xj.y), rz = fs(xi.z, xj.z);
+        const float s = dist2(rx, ry, rz);
+        if (!(s <= S.smax)) return;
+        const float4 vj = __ldg(sv + j), dj = __ldg(sd + j);
+        if (FM)
+            force_pair_fast(S, acc, rx, ry, rz, dist2_fma(rx, ry, rz), vi.x, vi.y, vi.z, di.y, vj, dj.y, dj.z,
+                            __float_as_int(xj.w), (int)j == pl);
+        else
+            force_pair(S, acc, rx, ry, rz, fsq(s), vi.x, vi.y, vi.z, di.y, vj, dj.y, dj.z, __float_as_int(xj.w),
+                       (int)j == pl);
+    });
+}
+
+// force over the packed records: the list walk of k_force taken two
+// neighbours at a time, in warp slices from the counter.  The L1 data path
+// bounds it: a gather of 32 records from a few cells costs about 24 of its
+// cycles, 71% of the fast form's time; taking neighbours in pairs cut the
+// other part, the instructions (227 to 137 million a launch at 1,048,576
+// particles, 56 in range), and with them the time from 351 to 270 us (exact
+// arithmetic 447 to 364, with the packed records in place of three arrays).
+// The fast form loads the records of the next pair before it sums the current
+// one, at 80 registers and 24 warps an SM (without: 281 us at 64 registers,
+// 309 at 80); the exact form, with more arithmetic between its loads, is
+// faster with 32 warps and no records in flight (364 vs 375 us).
+template <bool FM, bool REC>
+__global__ void __launch_bounds__(kMaxTile, FM ? 3 : 4) k_force_rec(const __grid_constant__ DevArrays a) {
+    const int nwork = *a.n_ptiles;
+    const int spt = a.tile / 32;
+    for (int sl = first_slice<true>(a.ctr + 1); sl < nwork * spt; sl = next_slice<true>(a.ctr + 1, sl)) {
+        const int w = sl / spt;
+        const int li = (sl % spt) * 32 + (int)(threadIdx.x & 31);
+        const Work wk = a.ptiles[w];
+        if (a.steps_left[wk.scene] == 0) continue;
+        const SceneDev& S = a.scenes[wk.scene];
+        if ((S.flags & kFlagOrdered) != 0) continue;
+        const int p = wk.start + li;
+        if (p >= S.p_off + S.n) continue;
+        const uint32_t pl = (uint32_t)(p - S.p_off);
+        ForceAcc acc = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, -1, 0};
+        const int cnt = a.ncnt[p];
+        if (cnt <= kNbCap) {
+            const float4* fd = a.fdat + 2 * (size_t)S.p_off;
+            const uint32_t* nl = a.nlist + (size_t)wk.start * kNbCap + li;
+            const int stride = a.tile;
+            const PairConst K = {S.h, S.hh, FM ? 3.0f * S.hh : fm(fm(3.0f, S.h), S.h), S.c_grad, S.c_spiky, S.mass,
+                                 FM ? S.cthr * S.cthr : S.cthr};
+            // pairs closer than the threshold (with a margin) take the general
+            // form, and so do all pairs of a particle whose own velocity or
+            // factors are not finite (zero times those is not zero)
+            const Rec me = ld_rec(fd + 2 * pl);
+            const float nxi = -lo(me.xy), nyi = -hi(me.xy), nzi = -lo(me.zA), Ai = hi(me.zA);
+            const float nvx = -lo(me.vxy), nvy = -hi(me.vxy), nvz = -lo(me.vzB);
+            const bool odd = !((nvx + nvy + nvz) * 0.0f + (Ai + hi(me.vzB)) * 0.0f == 0.0f);
+            const float c2 = odd ? INFINITY : S.cthr * S.cthr * 1.0001f;
+            const bool rec = REC && (S.flags & kFlagRecord) != 0;
+            uint32_t j0 = pl, j1 = pl, k0 = pl, k1 = pl;  // past the end: the particle itself
+            if (0 < cnt) j0 = __ldg(nl);
+            if (1 < cnt) j1 = __ldg(nl + stride);
+            if (2 < cnt) k0 = __ldg(nl + 2 * stride);
+            if (3 < cnt) k1 = __ldg(nl + 3 * stride);
+            nl += 4 * stride;
+            Rec ra, rb;
+            if (FM) {
+                ra = ld_rec(fd + 2 * j0);
+                rb = ld_rec(fd + 2 * j1);
+            }
+            for (int q = 0; q < cnt; q += 2) {
+                if (!FM) {
+                    ra = ld_rec(fd + 2 * j0);
+                    rb = ld_rec(fd + 2 * j1);
+                }
+                const PairIn A = pair_in<FM>(ra, nxi, nyi, nzi, Ai, nvx, nvy, nvz);
+                const PairIn B = pair_in<FM>(rb, nxi, nyi, nzi, Ai, nvx, nvy, nvz);
+                if (FM) {
+                    ra = ld_rec(fd + 2 * k0);
+                    rb = ld_rec(fd + 2 * k1);
+                }
+                bool general = false;
+                if (fminf(A.s, B.s) < c2) general = odd || (A.s < c2 && j0 != pl) || (B.s < c2 && j1 != pl);
+                if (REC && rec) {
+                    const float4* sp = a.spos + S.p_off;
+                    if (j0 != pl) acc.nb = max(acc.nb, __float_as_int(__ldg(&sp[j0].w))), acc.any = 1;
+                    if (j1 != pl) acc.nb = max(acc.nb, __float_as_int(__ldg(&sp[j1].w))), acc.any = 1;
+                }
+                const bool two = q + 1 < cnt;
+                if (!general) {
+                    force_two<FM>(K, acc, A, B, two ? B.B : 0.0f);
+                } else {
+                    force_one<FM>(S, acc, A, j0 == pl);
+                    if (two) force_one<FM>(S, acc, B, j1 == pl);
+                }
+                j0 = k0;
+                j1 = k1;
+                k0 = k1 = pl;
+                if (q + 4 < cnt) k0 = __ldg(nl);
+                if (q + 5 < cnt) k1 = __ldg(nl + stride);
+                nl += 2 * stride;
+            }
+        }
+        const float4 xi = a.spos[p];
+        const float4 vi = a.svel[p];
+        const float4 di = a.dyn[p];
+        if (cnt > kNbCap) {
+            ForceAcc walk = acc;
+            force_cells<FM>(a, S, p, walk);
+            acc = walk;
+        }
+        integrate_and_store(a, S, p, xi, vi, di.x, acc, true);
     }
 }
 
@@ -1732,7 +1969,7 @@ static size_t list_bytes(const LaunchShape& s) { return (size_t)kListCap * s.til
 // into one 32-byte record.
 template <int MINB, bool DYN, bool FM>
 static void launch_density_nl_d(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    const bool x2 = (s.variant & 64) != 0, pack = (s.variant & 128) != 0;
+    const bool x2 = (s.variant & 64) != 0, pack = s.pack;
     const int grid = DYN ? s.grid_dyn : s.grid_p;
     if (x2 && pack)
         k_density<false, false, MINB, true, true, true, DYN, FM><<<grid, s.tile, 0, st>>>(a);
@@ -1846,54 +2083,31 @@ void launch_force(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
         launch_force_coop(a, s, st);
         return;
     }
-    // the list variants walk their lists (or, on overflow, the cells) per
-    // lane and need no shared memory; bit 15 (32768) has the pipelined list
-    // walks take their work in warp slices from a counter (same bits)
-    const bool dyn = (s.variant & 32768) != 0;
+    // The list variants walk their lists (or, on overflow, the cells) per
+    // lane: over the packed records wherever the system holds them, since that
+    // form is the fastest at every size measured; warps take their work in
+    // slices from a counter.
     if ((s.variant & 262144) && (s.variant & (131072 | 128 | 24)) == (131072 | 128 | 24) && s.fmap) {
         // bit 18: the TMA gather pipeline (fast arithmetic, packed records)
         k_force_tma<3><<<s.grid_p, s.tile + 32, force_tma_smem(s.tile), st>>>(a, *static_cast<const CUtensorMap*>(s.fmap));
         return;
     }
-    if ((s.variant & 131072) && (s.variant & 24) == 24) {
-        // bit 17: fast arithmetic (force_pair_fast), pipelined list walk
-        const bool pack = (s.variant & 128) != 0;
-        if (pack) {
-            if (dyn)
-                k_force<false, 4, 3, true, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
+    if (s.variant & 8) {
+        const bool fast = (s.variant & (131072 | 16)) == (131072 | 16);
+        if (!s.pack) {
+            if (fast)
+                k_force<false, 4, true, true, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
             else
-                k_force<false, 4, 3, false, true><<<s.grid_p, s.tile, 0, st>>>(a);
-        } else if (dyn)
-            k_force<false, 4, 2, true, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
-        else
-            k_force<false, 4, 2, false, true><<<s.grid_p, s.tile, 0, st>>>(a);
-        return;
-    }
-    if ((s.variant & 136) == 136) {
-        if (dyn) {
-            if (s.variant & 4)
-                k_force<false, 3, 3, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
+                k_force<false, 4, true, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
+        } else if (s.record) {
+            if (fast)
+                k_force_rec<true, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
             else
-                k_force<false, 4, 3, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
-        } else if (s.variant & 4)
-            k_force<false, 3, 3><<<s.grid_p, s.tile, 0, st>>>(a);
+                k_force_rec<false, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
+        } else if (fast)
+            k_force_rec<true, false><<<s.grid_dyn, s.tile, 0, st>>>(a);
         else
-            k_force<false, 4, 3><<<s.grid_p, s.tile, 0, st>>>(a);
-    } else if ((s.variant & 24) == 24) {
-        if (dyn) {
-            if (s.variant & 4)
-                k_force<false, 3, 2, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
-            else
-                k_force<false, 4, 2, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
-        } else if (s.variant & 4)
-            k_force<false, 3, 2><<<s.grid_p, s.tile, 0, st>>>(a);
-        else
-            k_force<false, 4, 2><<<s.grid_p, s.tile, 0, st>>>(a);
-    } else if (s.variant & 8) {
-        if (s.variant & 4)
-            k_force<false, 3, 1><<<s.grid_p, s.tile, 0, st>>>(a);
-        else
-            k_force<false, 4, 1><<<s.grid_p, s.tile, 0, st>>>(a);
+            k_force_rec<false, false><<<s.grid_dyn, s.tile, 0, st>>>(a);
     } else if (s.variant & 4)
         k_force<false, 3><<<s.grid_p, s.tile, list_bytes(s), st>>>(a);
     else

@@ -48,8 +48,8 @@ struct DevArrays {
     // kNbCap: that particle's force pass then walks the cells).
     uint32_t* nlist;
     int32_t* ncnt;
-    // packed neighbour records (variant bit 7), two float4 per sorted
-    // particle: (x, y, z, P/rho^2) and (vx, vy, vz, m/rho)
+    // packed neighbour records, two float4 per sorted particle:
+    // (x, y, z, P/rho^2) and (vx, vy, vz, m/rho)
     float4* fdat;
     // status word: bit 0 = ordered-mode neighbour overflow, bit 1 =
     // inconsistent sort counts, bit 2 = a bounded wait of the TMA force
@@ -71,6 +71,8 @@ struct LaunchShape {
     int grid_c;      // persistent grid of the scan
     int grid_t;      // persistent grid of the terrain kernel
     int variant;     // sph_system_config.variant bits (bit 3 only with lists allocated)
+    bool pack;       // the density pass writes packed records, the force pass gathers them
+    bool record;     // some scene keeps its force records (SPH_FLAG_RECORD)
     int grid_dyn;    // grid of the dynamically scheduled neighbour kernels
     const void* fmap;  // host copy of the CUtensorMap over the packed records (null: none)
 };

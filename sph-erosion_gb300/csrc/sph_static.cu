@@ -189,6 +189,8 @@ extern "C" SPH_API int sph_density_static(const sph_params* p, int n, const floa
         s.grid_c = (int)ct.size();
         s.grid_t = 0;
         s.variant = 0;
+        s.pack = false;
+        s.record = false;
         s.grid_dyn = 0;
         s.fmap = nullptr;
 
