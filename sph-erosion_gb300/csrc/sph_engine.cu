@@ -1200,6 +1200,7 @@ LaunchShape System::shape() const {
     s.grid_t = n_ttiles_;
     s.variant = nl_ready_ ? cfg_.variant : (cfg_.variant & ~504);
     s.record = any_record_;
+    group_rules(s);
     s.pack = nl_ready_ && fdat_.n > 0;
     // enough blocks to fill every SM (2048 threads each); blocks that start
     // after the counter ran out exit at once

@@ -461,17 +461,17 @@ __device__ __forceinline__ void force_pair_fast(const SceneDev& S, ForceAcc& acc
     if (s < S.cthr * S.cthr) {
         // coincident: gradPressure along normalize(1, 1, 1)
         const float hl = S.h - sqrtf(s);
-        const float g = -(S.inv_sqrt3 * S.c_spiky) * (hl * hl) * coef;
-        acc.fpx += g;
-        acc.fpy += g;
-        acc.fpz += g;
+        const float t = -(S.inv_sqrt3 * S.c_spiky) * (hl * hl);
+        acc.fpx = fmaf(t, coef, acc.fpx);
+        acc.fpy = fmaf(t, coef, acc.fpy);
+        acc.fpz = fmaf(t, coef, acc.fpz);
         const float bl = Bj * (S.c_spiky * hl);
         acc.fvx = fmaf(vj.x - vix, bl, acc.fvx);
         acc.fvy = fmaf(vj.y - viy, bl, acc.fvy);
         acc.fvz = fmaf(vj.z - viz, bl, acc.fvz);
     } else {
         const float inv = rsqrtf(s);  // 1/|r|
-        const float hl = S.h - s * inv;  // h - |r|
+        const float hl = fmaf(-s, inv, S.h);  // h - |r|
         const float g = -(S.c_spiky * coef) * (hl * hl) * inv;  // gradPressure / |r|, times coef
         acc.fpx = fmaf(rx, g, acc.fpx);
         acc.fpy = fmaf(ry, g, acc.fpy);
@@ -1562,6 +1562,305 @@ __global__ void __launch_bounds__(256, MINB) k_force_coop(DevArrays a) {
 }
 
 // ---------------------------------------------------------------------------
+// Neighbour passes for small systems: a group of G lanes per particle, as in
+// the cooperative passes, but with every sum taken in list order, so that the
+// results are the per-lane passes' bit for bit.  With one particle per lane a
+// system of a few thousand particles is a few dozen warps, each walking its
+// rows and lists as one chain of dependent loads; here the chain is one row
+// table and a few windows of G candidates long.  The terms of a window are
+// computed by all lanes and left in shared memory in order; the sequential
+// additions, four cycles each, are then the only serial part, and one lane per
+// particle does them and the per-particle arithmetic for the whole block.  All
+// this takes about three times the per-lane passes' instructions, so it is for
+// systems of few particles (group_rules).  Density and force, us, exact
+// arithmetic: 1,000 particles 27 + 19 -> 10 + 10, 16,384 48 + 34 -> 25 + 20.
+// Group number `slot` takes lane slot % T of work tile slot / T.
+constexpr int kTerms = 256;  // density terms a group holds before it adds them
+
+template <int G, int R, bool FM>
+__device__ __forceinline__ void density_group_particle(const DevArrays& a, const SceneDev& S, int p, uint32_t* nl,
+                                                       int stride, int* soff, float* term, const Group<G>& g,
+                                                       int& count, int& left, float& part) {
+    const float4 xi = a.spos[p];
+    const Probe q = probe_of(S, xi);
+    constexpr int XS = R == 1 ? 2 : 1;  // the scene's xsub at this reach
+    constexpr int RX = (R > 0 ? R : 1) * XS;
+    float gx2[2 * RX + 1];  // squared x-gaps in y/z cell units
+    if (R > 0) {
+#pragma unroll
+        for (int d = -RX; d <= RX; ++d) {
+            const int k = q.c.cx + d;
+            float g2 = INFINITY;
+            if (k >= 0 && k < S.nx) {
+                const float gg = cell_gap(q.tx, k, S.nx) * (1.0f / XS);
+                g2 = gg * gg;
+            }
+            gx2[d + RX] = g2;
+        }
+    }
+    const float4* sp = a.spos + S.p_off;
+    const int side = R > 0 ? 2 * R + 1 : 2 * S.reach + 1;
+    const int nrows = side * side;
+    const float mc = S.mass * S.c_poly6;
+    float rho = 0.0f;
+    int cnt = 0, done = 0;  // in-range candidates, terms added
+    auto make_terms = [&]() {  // squared distances to terms
+        __syncwarp(g.mask);
+        for (int k = g.gl; k < cnt - done; k += G) {
+            const float hs = S.hh - term[k];
+            term[k] = FM ? hs * hs * hs : density_term(S, fsq(term[k]));
+        }
+    };
+    auto add_terms = [&]() {
+        make_terms();
+        __syncwarp(g.mask);
+        for (int k = 0; k < cnt - done; ++k) rho = FM ? fmaf(mc, term[k], rho) : fa(rho, term[k]);
+        done = cnt;
+        __syncwarp(g.mask);
+    };
+    const unsigned below = (1u << g.gl) - 1u;
+    for (int rb = 0; rb < nrows; rb += G) {
+        uint32_t st = 0, en = 0;
+        if (rb + g.gl < nrows) stencil_row<R>(a, S, q, gx2, rb + g.gl, st, en);
+        const int len = (int)(en - st);
+        int inc = len;
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+            const int v = __shfl_up_sync(g.mask, inc, o, G);
+            if (g.gl >= o) inc += v;
+        }
+        const int pre = inc - len;
+        const int total = __shfl_sync(g.mask, inc, G - 1, G);
+        int carry = 0;
+        for (int wb = 0; wb < total; wb += G) {
+            // the rows that start in this window record where their
+            // candidates sit: candidate t of the stream is particle t + off
+            const bool starts = len > 0 && pre >= wb && pre < wb + G;
+            if (starts) soff[pre - wb] = (int)st - pre;
+            const unsigned m = __reduce_or_sync(g.mask, starts ? (1u << (pre - wb)) : 0u);
+            __syncwarp(g.mask);
+            const unsigned upto = m & ((2u << g.gl) - 1u);
+            const int off = upto ? soff[31 - __clz(upto)] : carry;
+            carry = m ? soff[31 - __clz(m)] : carry;
+            __syncwarp(g.mask);
+            const int t = wb + g.gl;
+            bool in = false;
+            uint32_t j = 0;
+            float s = 0.0f;
+            if (t < total) {
+                j = (uint32_t)(t + off);
+                const float4 xj = __ldg(sp + j);
+                s = dist2(fs(xi.x, xj.x), fs(xi.y, xj.y), fs(xi.z, xj.z));
+                in = s <= S.smax;
+            }
+            if (cnt - done > kTerms - G) add_terms();
+            const unsigned b = (__ballot_sync(g.mask, in) & g.mask) >> g.gbase;
+            const int at = cnt + __popc(b & below);
+            if (in) {
+                if (nl && at < kNbCap) nl[(size_t)at * stride] = j;
+                term[at - done] = s;
+            }
+            cnt += __popc(b);
+        }
+    }
+    make_terms();
+    count = cnt;
+    left = cnt - done;
+    part = rho;
+}
+
+// lane_lists: the lists (and the packed records) go to a per-lane force pass;
+// else a list's entries are together, for k_force_group.  Each warp takes one
+// particle; one lane for each of the block's particles then adds its terms and
+// finishes it.
+template <bool FM>
+__global__ void __launch_bounds__(256, 5) k_density_group(const __grid_constant__ DevArrays a, bool lane_lists,
+                                                          bool pack) {
+    constexpr int G = 32, N = 256 / G;
+    __shared__ int s_off[256];
+    __shared__ float s_term[N][kTerms + 1];
+    __shared__ int s_p[N], s_cnt[N], s_left[N];
+    __shared__ float s_part[N];
+    const Group<G> g;
+    const int wid = threadIdx.x / G, slot = (int)blockIdx.x * N + wid, w = slot / a.tile, l = slot % a.tile;
+    Work wk = {0, 0};
+    int p = -1;
+    if (w < *a.n_ptiles) {
+        wk = a.ptiles[w];
+        const SceneDev& S = a.scenes[wk.scene];
+        if (a.steps_left[wk.scene] != 0 && !(S.flags & kFlagOrdered) && wk.start + l < S.p_off + S.n) p = wk.start + l;
+    }
+    const SceneDev& S = a.scenes[wk.scene];  // the tile's, the same for the whole block
+    if (p >= 0) {
+        int* soff = s_off + (threadIdx.x & ~(G - 1));
+        float* term = s_term[wid];
+        const int stride = lane_lists ? a.tile : 1;
+        uint32_t* nl = a.nlist ? a.nlist + (lane_lists ? (size_t)wk.start * kNbCap + l : (size_t)p * kNbCap) : nullptr;
+        int cnt, left;
+        float part;
+        if (S.reach == 1)
+            density_group_particle<G, 1, FM>(a, S, p, nl, stride, soff, term, g, cnt, left, part);
+        else if (S.reach == 2)
+            density_group_particle<G, 2, FM>(a, S, p, nl, stride, soff, term, g, cnt, left, part);
+        else
+            density_group_particle<G, 0, FM>(a, S, p, nl, stride, soff, term, g, cnt, left, part);
+        if (g.gl == 0) s_cnt[wid] = cnt, s_left[wid] = left, s_part[wid] = part;
+    }
+    if (g.gl == 0) s_p[wid] = p;
+    __syncthreads();
+    const int q = threadIdx.x;
+    if (q >= N || s_p[q] < 0) return;
+    p = s_p[q];
+    const float mc = S.mass * S.c_poly6;
+    float rho = s_part[q];
+    for (int k = 0; k < s_left[q]; ++k) rho = FM ? fmaf(mc, s_term[q][k], rho) : fa(rho, s_term[q][k]);
+    const float P = fm(S.k, fs(rho, S.p0));
+    const float Ai = fdv(P, fm(rho, rho)), Bi = fdv(S.mass, rho);
+    a.dyn[p] = make_float4(rho, Ai, Bi, P);
+    if (a.ncnt) a.ncnt[p] = s_cnt[q];
+    if (pack) {
+        const float4 xi = a.spos[p], vi = a.svel[p];
+        a.fdat[2 * (size_t)p] = make_float4(xi.x, xi.y, xi.z, Ai);
+        a.fdat[2 * (size_t)p + 1] = make_float4(vi.x, vi.y, vi.z, Bi);
+    }
+}
+
+// Values a lane leaves for the ordered sums of one pair.  Exact arithmetic:
+// the ten addends (pressure, viscosity, normal, colour field).  Fast: the
+// factors of the ten fused multiply-adds: the pressure direction, r, the
+// velocity difference, then g, b, gn, m/rho_j and the Laplacian.
+template <bool FM>
+constexpr int kPairValues = FM ? 14 : 10;
+
+template <bool FM>
+__device__ __forceinline__ void pair_values(const SceneDev& S, float rx, float ry, float rz, float vx, float vy, float vz,
+                                            float AA, float Bj, bool self, float* v) {
+#pragma unroll
+    for (int c = 0; c < kPairValues<FM>; ++c) v[c] = 0.0f;  // the particle itself adds to the colour field only
+    if (FM) {
+        const float s = dist2_fma(rx, ry, rz);
+        const float hs = S.hh - s;
+        v[12] = Bj;
+        v[13] = (-S.c_grad * hs) * fmaf(-7.0f, s, 3.0f * S.hh);
+        if (self) return;
+        const float coef = AA * S.mass;
+        if (s < S.cthr * S.cthr) {
+            const float hl = S.h - sqrtf(s);
+            const float t = -(S.inv_sqrt3 * S.c_spiky) * (hl * hl);
+            v[0] = v[1] = v[2] = coef;
+            v[9] = t;
+            v[10] = Bj * (S.c_spiky * hl);
+        } else {
+            const float inv = rsqrtf(s);
+            const float hl = fmaf(-s, inv, S.h);
+            v[0] = rx, v[1] = ry, v[2] = rz;
+            v[9] = -(S.c_spiky * coef) * (hl * hl) * inv;
+            v[10] = Bj * (S.c_spiky * hl);
+        }
+        v[3] = rx, v[4] = ry, v[5] = rz;
+        v[6] = vx, v[7] = vy, v[8] = vz;
+        v[11] = -(Bj * S.c_grad) * (hs * hs);
+    } else {
+        // one pair from zero sums: 0 + x is x (a zero's sign aside)
+        ForceAcc one = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, -1, 0};
+        force_pair(S, one, rx, ry, rz, fsq(dist2(rx, ry, rz)), 0.f, 0.f, 0.f, AA, make_float4(vx, vy, vz, 0.f), 0.f, Bj,
+                   -1, self);
+        v[0] = one.fpx, v[1] = one.fpy, v[2] = one.fpz;
+        v[3] = one.fvx, v[4] = one.fvy, v[5] = one.fvz;
+        v[6] = one.nx, v[7] = one.ny, v[8] = one.nz;
+        v[9] = one.cfl;
+    }
+}
+
+template <bool FM, bool REC>
+__global__ void __launch_bounds__(256, 4) k_force_group(const __grid_constant__ DevArrays a) {
+    constexpr int G = 16, N = 256 / G, V = kPairValues<FM>, W = G + 1;
+    __shared__ float s_val[N][V][W];
+    __shared__ float s_sum[N][13];  // the ten sums, NeighbId, whether there is a neighbour; the particle
+    const Group<G> g;
+    const int grp = threadIdx.x / G, slot = (int)blockIdx.x * N + grp, w = slot / a.tile;
+    float(*val)[W] = s_val[grp];
+    float* sum = s_sum[grp];
+    Work wk = {0, 0};
+    int p = -1;
+    if (w < *a.n_ptiles) {
+        wk = a.ptiles[w];
+        const SceneDev& S = a.scenes[wk.scene];
+        const int at = wk.start + slot % a.tile;
+        if (a.steps_left[wk.scene] != 0 && !(S.flags & kFlagOrdered) && at < S.p_off + S.n) p = at;
+    }
+    const SceneDev& S = a.scenes[wk.scene];  // the tile's, the same for the whole block
+    const int cnt = p >= 0 ? a.ncnt[p] : 0;
+    int nb = -1, any = 0;
+    if (p < 0) {
+    } else if (cnt > kNbCap) {  // the list overflowed: one lane walks the cells
+        if (g.gl == 0) {
+            ForceAcc acc = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, -1, 0};
+            force_cells<FM>(a, S, p, acc);
+            sum[0] = acc.fpx, sum[1] = acc.fpy, sum[2] = acc.fpz;
+            sum[3] = acc.fvx, sum[4] = acc.fvy, sum[5] = acc.fvz;
+            sum[6] = acc.nx, sum[7] = acc.ny, sum[8] = acc.nz;
+            sum[9] = acc.cfl;
+            nb = acc.nb, any = acc.any;
+        }
+    } else {
+        const float4 xi = a.spos[p], vi = a.svel[p];
+        const float Ai = a.dyn[p].y;
+        const uint32_t pl = (uint32_t)(p - S.p_off);
+        const float4* sp = a.spos + S.p_off;
+        const float4* sv = a.svel + S.p_off;
+        const float4* sd = a.dyn + S.p_off;
+        const uint32_t* nl = a.nlist + (size_t)p * kNbCap;
+        // the two factors (or the addend) of this lane's sum
+        const int c = g.gl;
+        const int i1 = FM ? (c < 3 ? c : c < 6 ? c + 3 : c < 9 ? c - 3 : 12) : c;
+        const int i2 = c < 3 ? 9 : c < 6 ? 10 : c < 9 ? 11 : 13;
+        float acc = 0.0f;
+        uint32_t j = c < cnt ? __ldg(nl + c) : pl;
+        for (int b = 0; b < cnt; b += G) {
+            const float4 xj = __ldg(sp + j), vj = __ldg(sv + j), dj = __ldg(sd + j);
+            const bool live = b + c < cnt, self = j == pl;
+            if (REC && live && !self) nb = max(nb, __float_as_int(xj.w)), any = 1;
+            if (b + G + c < cnt) j = __ldg(nl + b + G + c);
+            if (live) {
+                float v[V];
+                pair_values<FM>(S, fs(xi.x, xj.x), fs(xi.y, xj.y), fs(xi.z, xj.z), fs(vj.x, vi.x), fs(vj.y, vi.y),
+                                fs(vj.z, vi.z), fa(Ai, dj.y), dj.z, self, v);
+#pragma unroll
+                for (int k = 0; k < V; ++k) val[k][c] = v[k];
+            }
+            __syncwarp(g.mask);
+            if (c < 10) {
+                const int m = min(G, cnt - b);
+                for (int k = 0; k < m; ++k) acc = FM ? fmaf(val[i1][k], val[i2][k], acc) : fa(acc, val[i1][k]);
+            }
+            __syncwarp(g.mask);
+        }
+        if (REC) {
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) {
+                nb = max(nb, __shfl_xor_sync(g.mask, nb, o, G));
+                any |= __shfl_xor_sync(g.mask, any, o, G);
+            }
+        }
+        if (c < 10) sum[c] = acc;
+    }
+    if (g.gl == 0) {
+        sum[10] = __int_as_float(nb), sum[11] = __int_as_float(any);
+        sum[12] = __int_as_float(p);
+    }
+    // one lane for each of the block's particles: the rest of the step
+    __syncthreads();
+    if (threadIdx.x >= N) return;
+    sum = s_sum[threadIdx.x];
+    p = __float_as_int(sum[12]);
+    if (p < 0) return;
+    const ForceAcc acc = {sum[0], sum[1], sum[2], sum[3], sum[4], sum[5], sum[6], sum[7], sum[8], sum[9],
+                          __float_as_int(sum[10]), __float_as_int(sum[11])};
+    integrate_and_store(a, S, p, a.spos[p], a.svel[p], a.dyn[p].x, acc, true);
+}
+
+// ---------------------------------------------------------------------------
 // Force pass with a TMA gather pipeline (variant bit 18, with lists, packed
 // records and fast arithmetic).  Each block holds T consumer threads (one
 // particle of the tile each) and one producer warp.  For list slot q the
@@ -2048,6 +2347,45 @@ static void launch_force_coop(const DevArrays& a, const LaunchShape& s, cudaStre
         launch_force_coop_b<4>(a, s, st);
 }
 
+static void launch_density_group(const DevArrays& a, const LaunchShape& s, bool fast, cudaStream_t st) {
+    const int blocks = s.grid_p * s.tile / 8;
+    const bool lane_lists = !s.force_group, pack = lane_lists && s.pack;
+    if (fast)
+        k_density_group<true><<<blocks, 256, 0, st>>>(a, lane_lists, pack);
+    else
+        k_density_group<false><<<blocks, 256, 0, st>>>(a, lane_lists, pack);
+}
+
+static void launch_force_group(const DevArrays& a, const LaunchShape& s, bool fast, cudaStream_t st) {
+    const int blocks = s.grid_p * s.tile / 16;
+    if (s.record) {
+        if (fast)
+            k_force_group<true, true><<<blocks, 256, 0, st>>>(a);
+        else
+            k_force_group<false, true><<<blocks, 256, 0, st>>>(a);
+    } else if (fast)
+        k_force_group<true, false><<<blocks, 256, 0, st>>>(a);
+    else
+        k_force_group<false, false><<<blocks, 256, 0, st>>>(a);
+}
+
+// Which passes of a step take a group of lanes per particle: the per-lane list
+// forms (bit 8 without 256) of systems small enough to leave the chip idle with
+// one lane per particle.  The lines are where the group passes stop paying
+// when three systems run at once on streams of their own, which fills the chip
+// first (us a step, group vs per lane; settled pools): exact arithmetic, both
+// passes, 12,000 particles 26.8 vs 34.0, 16,000 32.4 vs 36.1, 20,000 40.6 vs
+// 38.3; fast, density 8,000 19.7 vs 24.1, 12,000 24.5 vs 25.7, 16,000 29.0 vs
+// 27.1; fast, force (beside the group density pass) 8,000 19.1 vs 19.7, 12,000
+// 26.5 vs 24.5.  A system alone on the chip gains up to there from 2.3x (1,000
+// particles: 74 to 32 us) to 1.6x (20,000: 99 to 62 us) a step.
+void group_rules(LaunchShape& s) {
+    const int64_t n = (int64_t)s.grid_p * s.tile;
+    const bool lists = (s.variant & (8 | 256)) == 8;
+    s.density_group = lists && n <= ((s.variant & 131072) ? 12288 : 18432);
+    s.force_group = s.density_group && n <= ((s.variant & (131072 | 16)) == (131072 | 16) ? 8192 : 18432);
+}
+
 static bool coop(const LaunchShape& s) { return (s.variant & (256 | 8)) == (256 | 8); }
 
 void launch_density(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
@@ -2056,7 +2394,9 @@ void launch_density(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
         return;
     }
     const bool relaxed = (s.variant & 4) != 0;
-    if (s.variant & 8) {
+    if (s.density_group) {
+        launch_density_group(a, s, (s.variant & 131072) != 0, st);
+    } else if (s.variant & 8) {
         if (relaxed)
             launch_density_nl<4>(a, s, st);
         else if (s.variant & 32)
@@ -2083,11 +2423,15 @@ void launch_force(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
         launch_force_coop(a, s, st);
         return;
     }
+    if (s.force_group) {
+        launch_force_group(a, s, (s.variant & (131072 | 16)) == (131072 | 16), st);
+        return;
+    }
     // The list variants walk their lists (or, on overflow, the cells) per
     // lane: over the packed records wherever the system holds them, since that
     // form is the fastest at every size measured; warps take their work in
     // slices from a counter.
-    if ((s.variant & 262144) && (s.variant & (131072 | 128 | 24)) == (131072 | 128 | 24) && s.fmap) {
+    if (!s.force_group && (s.variant & 262144) && (s.variant & (131072 | 128 | 24)) == (131072 | 128 | 24) && s.fmap) {
         // bit 18: the TMA gather pipeline (fast arithmetic, packed records)
         k_force_tma<3><<<s.grid_p, s.tile + 32, force_tma_smem(s.tile), st>>>(a, *static_cast<const CUtensorMap*>(s.fmap));
         return;

@@ -183,6 +183,7 @@ extern "C" SPH_API int sph_density_static(const sph_params* p, int n, const floa
         a.chunk_sum = reinterpret_cast<uint32_t*>(base + kOffChunk);
         a.tab = reinterpret_cast<const uint32_t*>(base + kOffTab);
         a.status = reinterpret_cast<unsigned*>(base + kOffStatus);
+        a.tile = kStaticTile;
         LaunchShape s;
         s.tile = kStaticTile;
         s.grid_p = (int)pt.size();
@@ -190,6 +191,8 @@ extern "C" SPH_API int sph_density_static(const sph_params* p, int n, const floa
         s.grid_t = 0;
         s.variant = 0;
         s.pack = false;
+        s.density_group = true;  // at most 32,768 particles (group_rules)
+        s.force_group = true;    // no list is written
         s.record = false;
         s.grid_dyn = 0;
         s.fmap = nullptr;

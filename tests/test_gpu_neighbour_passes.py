@@ -2,17 +2,24 @@
 wrong: bit for bit the pass that walks the cells (exact arithmetic) and the
 shared-memory gather pipeline (fast arithmetic), which share no list walk with
 them."""
+import functools
+
 import numpy as np
 import pytest
 
 import sph_gb300 as S
-from helpers import REF, run
+from helpers import REF
 
 pytestmark = pytest.mark.gpu
 
 # particles of a cluster = in-range neighbours of each of them, itself included;
-# around the pairs, quads and rings of four of the walks and the list's 192
+# around the pairs, quads and windows of 16 of the walks and the list's 192
 SIZES = [1, 2, 3, 4, 5, 7, 8, 9, 12, 13, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 191, 192, 193, 200]
+# particles of a second scene in the system: with 0 both passes take a group of
+# lanes per particle, with 8,000 the fast force pass takes one lane, with 14,000
+# the fast density pass too, with 20,000 all do
+FILL = [0, 8000, 14000, 20000]
+CELLS, GATHER = 0, 426232  # variants: cell walk; TMA gather pipeline
 
 
 def clusters(rng, sizes, box=0.9, radius=0.006):
@@ -30,6 +37,8 @@ def case(name):
     if name == "coincident":
         pos[5], pos[6], pos[7] = pos[4], pos[4], pos[8]
         vel[6] = vel[4]
+        k = rng.permutation(np.arange(100, len(pos)))[:600]  # and pairs nearer than 1e-4
+        pos[k[:300]] = pos[k[300:]] + rng.uniform(-5e-5, 5e-5, (300, 3))
     elif name == "infinite":
         vel[3, 1] = np.inf
         vel[10, 2] = -np.inf
@@ -37,18 +46,30 @@ def case(name):
     return pos, vel
 
 
-@pytest.mark.parametrize("cell_mult", [1.0, 0.5, 0.3])
-@pytest.mark.parametrize("name", ["plain", "coincident", "infinite"])
-def test_list_lengths_bit_exact(name, cell_mult):
+@functools.lru_cache(maxsize=None)
+def records(name, cell_mult, variant, fill, record=True, tile=256):
+    """Records after two steps of the clusters, beside `fill` other particles."""
     pos, vel = case(name)
-    prm = dict(REF, box_len=0.9)
-    for ref, forms in ((0, (88, 216)), (426232, (164088, 163960))):
-        want = run(prm, pos, 2, vel=vel, cell_mult=cell_mult, variant=ref)[2]
+    with S.System(particle_capacity=len(pos) + fill, variant=variant, tile=tile) as sysm:
+        prm = dict(REF, box_len=0.9, cell_mult=cell_mult, flags=S.SPH_FLAG_RECORD if record else 0)
+        sc = sysm.scene(S.default_params(**prm), capacity=len(pos))
+        sc.set_particles(pos, vel)
+        if fill:
+            other = sysm.scene(S.default_params(**dict(prm, flags=0)), capacity=fill)
+            other.set_particles(np.random.default_rng(1).uniform(-0.8, 0.8, (fill, 3)))
+        sysm.step(2)
+        return sc.get_records()
+
+
+@pytest.mark.parametrize("cell_mult", [1.0, 0.5, 0.3])
+@pytest.mark.parametrize("fill", FILL)
+@pytest.mark.parametrize("name", ["plain", "coincident", "infinite"])
+def test_list_lengths_bit_exact(name, fill, cell_mult):
+    for reference, forms in ((CELLS, (88, 216)), (GATHER, (164088, 163960))):
+        want = records(name, cell_mult, reference, FILL[-1])
         for v in forms:
-            for record in (True, False):
-                flags = S.SPH_FLAG_RECORD if record else 0
-                got = run(prm, pos, 2, vel=vel, cell_mult=cell_mult, variant=v, flags=flags)[2]
-                cols = slice(0, 27) if record else slice(0, 6)
-                assert np.array_equal(got[0][:, cols], want[0][:, cols], equal_nan=True), (ref, v, record)
-                if record:
-                    assert np.array_equal(got[1], want[1]), (ref, v)
+            got = records(name, cell_mult, v, fill)
+            assert np.array_equal(got[0], want[0], equal_nan=True), (reference, v)
+            assert np.array_equal(got[1], want[1]), (reference, v)
+        got = records(name, cell_mult, forms[0], fill, record=False, tile=128)
+        assert np.array_equal(got[0][:, :6], want[0][:, :6], equal_nan=True), reference
