@@ -78,12 +78,13 @@ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
     return r;
 }
 __device__ __forceinline__ f2 add2(f2 a, f2 b) { return fma2(a, pk(1.0f), b); }
-// A product that an addition follows, as a * b + (-0) with the -0 read from
-// memory: the assembler fuses mul.rn.f32x2 into an addition that uses its
-// result (also into a scalar one), which would drop the product's rounding;
-// this form it cannot fuse.
-__constant__ float kNegZero[2] = {-0.0f, -0.0f};
-__device__ __forceinline__ f2 mulr2(f2 a, f2 b) { return fma2(a, b, pk(kNegZero[0], kNegZero[1])); }
+// A product that an addition follows, as a * b + (-0) with a -0 that the
+// assembler does not know (neg_zero, read once per kernel): it fuses
+// mul.rn.f32x2 into an addition that uses its result (also into a scalar one),
+// which would drop the product's rounding; this form it cannot fuse.
+__constant__ float kNegZero = -0.0f;
+__device__ __forceinline__ f2 neg_zero() { return pk(*(volatile const float*)&kNegZero); }
+__device__ __forceinline__ f2 mulr2(f2 a, f2 b, f2 nz) { return fma2(a, b, nz); }
 
 // A packed neighbour record (DevArrays::fdat) as four pairs: (x, y),
 // (z, P/rho^2), (vx, vy), (vz, m/rho); one 256-bit load.
@@ -276,22 +277,6 @@ __device__ __forceinline__ void for_each_candidate(const DevArrays& a, const Sce
     });
 }
 
-// The same visit with the candidates of a row taken two at a time (both
-// loads issued before either is tested); the order is unchanged.
-template <class F>
-__device__ __forceinline__ void for_each_candidate_x2(const DevArrays& a, const SceneDev& S, float4 xi, F&& f) {
-    const float4* sp = a.spos + S.p_off;
-    for_rows(a, S, xi, true, [&](uint32_t st, uint32_t en) {
-        uint32_t j = st;
-        for (; j + 1 < en; j += 2) {
-            const float4 x0 = __ldg(sp + j), x1 = __ldg(sp + j + 1);
-            f(j, x0);
-            f(j + 1, x1);
-        }
-        if (j < en) f(j, __ldg(sp + j));
-    });
-}
-
 // In-range traversal of the fast path.  Candidates are tested in a tight
 // loop and the indices of in-range ones are compacted into a per-thread list
 // in shared memory (column threadIdx.x, so lanes touch distinct banks); the
@@ -441,11 +426,6 @@ __device__ __forceinline__ void force_pair(const SceneDev& S, ForceAcc& acc, flo
 // sum of squares.
 __device__ __forceinline__ float dist2_fma(float dx, float dy, float dz) {
     return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-}
-
-__device__ __forceinline__ float density_term_fast(const SceneDev& S, float s) {
-    const float hs = S.hh - s;
-    return (S.mass * S.c_poly6) * (hs * hs * hs);
 }
 
 __device__ __forceinline__ void force_pair_fast(const SceneDev& S, ForceAcc& acc, float rx, float ry, float rz,
@@ -780,6 +760,13 @@ __global__ void __launch_bounds__(kMaxTile) k_reorder(DevArrays a) {
     }
 }
 
+// Where entry q of the neighbour list of lane l of a tile of T particles is,
+// from the tile's start: groups of four entries, the lanes' groups side by
+// side.
+__device__ __forceinline__ uint32_t list_at(int q, int l, int T) {
+    return ((uint32_t)(q >> 2) * (uint32_t)T + (uint32_t)l) * 4u + (uint32_t)(q & 3);
+}
+
 // Work slices of the neighbour kernels.  Static: block b takes the tiles b,
 // b + gridDim.x, ..., and its thread t the tile's lane t.  Dynamic (DYN):
 // every warp takes the next 32-lane slice of any tile from a counter, so no
@@ -803,21 +790,16 @@ __device__ __forceinline__ int first_slice(unsigned* ctr) {
 // LISTED: the in-range pairs are compacted (for_each_in_range_listed) instead
 // of evaluated inside the candidate loop; which one is faster depends on the
 // neighbour density, so the autotuner picks it.
-template <bool ORDERED, bool LISTED, int MINB, bool NL = false, bool X2 = false, bool PACK = false,
-          bool DYN = false, bool FM = false>
+template <bool ORDERED, bool LISTED, int MINB>
 __global__ void __launch_bounds__(kMaxTile, MINB) k_density(DevArrays a) {
     extern __shared__ uint32_t list[];
     const int nwork = *a.n_ptiles;
-    const int spt = DYN ? a.tile / 32 : 1;  // slices per tile
-    for (int sl = first_slice<DYN>(a.ctr); sl < nwork * spt; sl = next_slice<DYN>(a.ctr, sl)) {
-        const int w = DYN ? sl / spt : sl;
-        const int li = DYN ? (sl % spt) * 32 + (int)(threadIdx.x & 31) : (int)threadIdx.x;  // lane within the tile
-        const int stride = DYN ? a.tile : (int)blockDim.x;
+    for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
         const Work wk = a.ptiles[w];
         if (a.steps_left[wk.scene] == 0) continue;
-        const SceneDev S = a.scenes[wk.scene];  // by value: the list stores cannot alias it
+        const SceneDev& S = a.scenes[wk.scene];
         if (((S.flags & kFlagOrdered) != 0) != ORDERED) continue;
-        const int p = wk.start + li;
+        const int p = wk.start + (int)threadIdx.x;
         const bool valid = p < S.p_off + S.n;
         if ((ORDERED || !LISTED) && !valid) continue;
         const float4 xi = a.spos[valid ? p : S.p_off];
@@ -837,34 +819,271 @@ __global__ void __launch_bounds__(kMaxTile, MINB) k_density(DevArrays a) {
             });
             if (!valid) continue;
         } else {
-            // NL: the in-range candidates, in visiting order, also go to the
-            // particle's neighbour list for the force pass
-            uint32_t* nl = a.nlist + (size_t)wk.start * kNbCap + li;
-            int cnt = 0;
-            auto visit = [&](uint32_t j, float4 xj) {
+            for_each_candidate(a, S, xi, [&](uint32_t, float4 xj) {
                 const float s = dist2(fs(xi.x, xj.x), fs(xi.y, xj.y), fs(xi.z, xj.z));
-                if (s <= S.smax) {
-                    if (FM)
-                        rho += density_term_fast(S, s);
-                    else
-                        rho = fa(rho, density_term(S, fsq(s)));
-                    if (NL) {
-                        if (cnt < kNbCap) nl[(size_t)cnt * stride] = j;
-                        ++cnt;
-                    }
-                }
-            };
-            if (X2) {
-                for_each_candidate_x2(a, S, xi, visit);
-            } else {
-                for_each_candidate(a, S, xi, visit);
-            }
-            if (NL) a.ncnt[p] = cnt;
+                if (s <= S.smax) rho = fa(rho, density_term(S, fsq(s)));
+            });
         }
         const float P = fm(S.k, fs(rho, S.p0));
         const float Ai = fdv(P, fm(rho, rho)), Bi = fdv(S.mass, rho);
         a.dyn[p] = make_float4(rho, Ai, Bi, P);
-        if (PACK) {
+    }
+}
+
+// dist2 of two candidates from the particle at (-nx, -ny, -nz), both at once.
+__device__ __forceinline__ f2 dist2_two(float4 x0, float4 x1, float nx, float ny, float nz, f2 nzero) {
+    const f2 dx = pk(fa(x0.x, nx), fa(x1.x, nx)), dy = pk(fa(x0.y, ny), fa(x1.y, ny)),
+             dz = pk(fa(x0.z, nz), fa(x1.z, nz));
+    return add2(add2(mulr2(dx, dx, nzero), mulr2(dy, dy, nzero)), mulr2(dz, dz, nzero));
+}
+
+// for_rows_r with its loads ahead of their use: while one row's candidates are
+// visited, the next row's two offsets and the row number of the one after are
+// on their way.
+template <int R, class Fn>
+__device__ __forceinline__ void for_rows_ahead(const DevArrays& a, const SceneDev& S, float4 xi, bool valid, Fn&& fn) {
+    const Probe q = probe_of(S, xi);
+    const uint32_t* off = a.offsets + S.k_off + q.c.cx;
+    const float H2 = S.hcell * S.hcell;
+    constexpr int XS = R == 1 ? 2 : 1, RX = R * XS, side = 2 * R + 1;
+    float gx2[2 * RX + 1];
+#pragma unroll
+    for (int d = -RX; d <= RX; ++d) {
+        const int k = q.c.cx + d;
+        float g2 = INFINITY;
+        if (k >= 0 && k < S.nx) {
+            const float g = cell_gap(q.tx, k, S.nx) * (1.0f / XS);
+            g2 = g * g;
+        }
+        gx2[d + RX] = g2;
+    }
+    const int nx = S.nx, ny = S.ny, nz = S.nz;
+    const uint32_t* tab = a.tab + S.tab_off;
+    int y = q.c.cy - R, z = q.c.cz - R;
+    float z2 = INFINITY;  // squared gap of slab z
+    auto slab = [&]() {
+        z2 = INFINITY;
+        if (valid && q.finite && z >= 0 && z < nz) {
+            const float g = cell_gap(q.tz, z, nz);
+            z2 = g * g;
+        }
+    };
+    slab();
+    uint32_t num = 0, st = 0, en = 0;  // row number; next range
+    int lohi = -1;                     // its cells (-1: not reached)
+#pragma unroll 1
+    for (int r = 0; r < side * side + 2; ++r) {
+        const uint32_t cst = st, cen = en;
+        st = en = 0;
+        if (lohi >= 0) {
+            const uint32_t* o = off + num * (uint32_t)nx;
+            st = __ldg(o - (lohi >> 4));
+            en = __ldg(o + (lohi & 15) + 1);
+        }
+        lohi = -1;
+        if (r < side * side) {
+            if (y >= 0 && y < ny) {
+                const float g = cell_gap(q.ty, y, ny);
+                const float r2 = H2 - g * g - z2;
+                if (r2 >= 0.0f) {
+                    int l = 0, h = 0;
+#pragma unroll
+                    for (int d = 1; d <= RX; ++d) {
+                        if (gx2[RX - d] <= r2) l = d;
+                        if (gx2[RX + d] <= r2) h = d;
+                    }
+                    lohi = l * 16 + h;
+                    num = __ldg(tab + z * ny + y);
+                }
+            }
+            if (++y > q.c.cy + R) {
+                y = q.c.cy - R;
+                ++z;
+                slab();
+            }
+        }
+        fn(cst, cen);
+    }
+}
+
+// Entries of a lane's buffer (ListOut).
+constexpr int kBuf = 24;
+
+// One lane's neighbour list while it is written.  The lanes of a warp are at
+// different entries, so an index stored by itself is four bytes to a sector of
+// its own: 61 million sectors a launch at 1,048,576 particles and cells of h,
+// half of the L1-to-L2 path's time, and L2 wrote some of them out half filled
+// (DRAM 406 MB written for 280).  Here the indices go to the lane's column of
+// a buffer in shared memory and from there to the list in groups of four, all
+// lanes together: 3,291 -> 2,719 us for the 8.4M rain in fast arithmetic.  24
+// entries a lane: 16 empty it too often (2,785), 40 leave the candidates too
+// little L1 (2,995).
+struct ListOut {
+    uint32_t* nl;      // the lane's group 0
+    uint32_t stride;   // words from one of its groups to the next
+    uint32_t* col;     // the lane's column
+    uint32_t* next;    // its first free entry
+    int flushed;
+
+    __device__ __forceinline__ int pending() const { return (int)(next - col) >> 5; }
+    __device__ __forceinline__ void add(uint32_t j) {
+        *next = j;
+        next += 32;
+    }
+    __device__ __forceinline__ void flush() {
+        int n = pending();
+        uint32_t* from = col;
+        for (; n >= 4; n -= 4, from += 128) {
+            const uint32_t e0 = from[0], e1 = from[32], e2 = from[64], e3 = from[96];
+            if (flushed < kNbCap) {
+                *reinterpret_cast<uint4*>(nl + (size_t)((uint32_t)(flushed >> 2) * stride)) = make_uint4(e0, e1, e2, e3);
+            }
+            flushed += 4;
+        }
+        if (from != col) {
+            if (n > 0) col[0] = from[0];
+            if (n > 1) col[32] = from[32];
+            if (n > 2) col[64] = from[64];
+            next = col + 32 * n;
+        }
+    }
+    __device__ __forceinline__ void make_room() {  // for four more in every lane
+        if (__any_sync(kFull, next > col + 32 * (kBuf - 4))) flush();
+    }
+    __device__ __forceinline__ int finish() {
+        const int cnt = flushed + pending();
+        while (flushed < cnt) {  // the last group may hold entries past the end
+            if (flushed < kNbCap)
+                *reinterpret_cast<uint4*>(nl + (size_t)((uint32_t)(flushed >> 2) * stride)) =
+                    make_uint4(col[0], col[32], col[64], col[96]);
+            flushed += 4;
+            col += 128;
+        }
+        return cnt;
+    }
+};
+
+// Tests the candidates [st, en) of a row, each lane its own, four at a time in
+// straight-line code: packed differences and squares, a compare each,
+// predicated appends of the in-range indices; with fast arithmetic also the
+// density term.  All lanes of the warp take part, for its longest row.
+template <bool FM>
+__device__ __forceinline__ void density_row(const SceneDev& S, const float4* sp, float nx, float ny, float nz, f2 nzero,
+                                            uint32_t st, uint32_t en, ListOut& out, float& rho) {
+    const float smax = S.smax, hh = S.hh, mc = S.mass * S.c_poly6;
+    auto hit = [&](bool in, uint32_t j, float c3) {
+        if (in) {
+            if (FM) rho = fmaf(mc, c3, rho);
+            out.add(j);
+        }
+    };
+    const int longest = __reduce_max_sync(kFull, (int)(en - st));
+    for (int t = 0; t < longest; t += 4) {
+        out.make_room();
+        const uint32_t j = st + t;
+        const bool m0 = j < en, m1 = j + 1 < en, m2 = j + 2 < en, m3 = j + 3 < en;
+        const float4* c = sp + j;
+        float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0, x2 = x0, x3 = x0;
+        if (m0) x0 = __ldg(c);
+        if (m1) x1 = __ldg(c + 1);
+        if (m2) x2 = __ldg(c + 2);
+        if (m3) x3 = __ldg(c + 3);
+        const f2 sa = dist2_two(x0, x1, nx, ny, nz, nzero), sb = dist2_two(x2, x3, nx, ny, nz, nzero);
+        f2 ca = 0, cb = 0;
+        if (FM) {
+            const f2 ha = fma2(sa, pk(-1.0f), pk(hh)), hb = fma2(sb, pk(-1.0f), pk(hh));
+            ca = mul2(mul2(ha, ha), ha);
+            cb = mul2(mul2(hb, hb), hb);
+        }
+        hit(m0 && lo(sa) <= smax, j, lo(ca));
+        hit(m1 && hi(sa) <= smax, j + 1, hi(ca));
+        hit(m2 && lo(sb) <= smax, j + 2, lo(cb));
+        hit(m3 && hi(sb) <= smax, j + 3, hi(cb));
+    }
+}
+
+// Sum of the exact density terms over a finished list, four entries at a time
+// with the next four loaded ahead; the cells again when the list overflowed.
+__device__ __forceinline__ float density_sum_exact(const DevArrays& a, const SceneDev& S, float4 xi, const uint32_t* nl,
+                                                   uint32_t stride, int cnt, f2 nzero) {
+    const float4* sp = a.spos + S.p_off;
+    float rho = 0.0f;
+    if (cnt > kNbCap) {
+        for_each_candidate(a, S, xi, [&](uint32_t, float4 xj) {
+            const float s = dist2(fs(xi.x, xj.x), fs(xi.y, xj.y), fs(xi.z, xj.z));
+            if (s <= S.smax) rho = fa(rho, density_term(S, fsq(s)));
+        });
+        return rho;
+    }
+    const float nx = -xi.x, ny = -xi.y, nz = -xi.z;
+    uint4 e = make_uint4(0, 0, 0, 0);
+    if (0 < cnt) e = *reinterpret_cast<const uint4*>(nl);
+    for (int q = 0; q < cnt; q += 4) {
+        nl += stride;
+        const uint32_t j[4] = {e.x, q + 1 < cnt ? e.y : e.x, q + 2 < cnt ? e.z : e.x, q + 3 < cnt ? e.w : e.x};
+        float4 x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = __ldg(sp + j[u]);
+        if (q + 4 < cnt) e = *reinterpret_cast<const uint4*>(nl);
+#pragma unroll
+        for (int u = 0; u < 4; u += 2) {
+            const f2 s2 = dist2_two(x[u], x[u + 1], nx, ny, nz, nzero);
+            const f2 l2 = pk(fsq(lo(s2)), fsq(hi(s2)));
+            // mass * (c * pow3(hh - len * len)), pow3 as above
+            const f2 v = fma2(mulr2(l2, l2, nzero), pk(-1.0f), pk(S.hh));
+            const f2 pp = mul2(v, v), w = fma2(v, v, mul2(pp, pk(-1.0f)));
+            const f2 c = mulr2(pp, v, nzero), f = fma2(pp, v, mul2(c, pk(-1.0f)));
+            const f2 t = mulr2(pk(S.mass), mul2(pk(S.c_poly6), add2(c, fma2(w, v, f))), nzero);
+            if (q + u < cnt) rho = fa(rho, lo(t));
+            if (q + u + 1 < cnt) rho = fa(rho, hi(t));
+        }
+    }
+    return rho;
+}
+
+// density with the neighbour lists (variant bit 3), one lane per particle.  The
+// fast arithmetic adds its short term in place; the exact form, whose term has
+// a square root, sums over the finished list, where every lane of the warp has
+// a pair to evaluate.  No unit bounds it (instructions 65%, L1 data path 60%):
+// the rows are walked in step, which keeps a warp's loads in few cache lines
+// but leaves 40% of the lanes waiting for the longest row.  80 registers: at 64
+// the compiler spills (fast 437 instead of 328 us), 16 warps an SM are too few
+// (392).  1,048,576 particles, before and after: fast, cells of h/2, 380 ->
+// 318 us; exact, cells of h, 488 -> 444 us.
+template <bool FM>
+__global__ void __launch_bounds__(kMaxTile, 3) k_density_list(const __grid_constant__ DevArrays a, bool pack) {
+    __shared__ uint32_t buf[kMaxTile / 32][kBuf][32];
+    const int nwork = *a.n_ptiles;
+    for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
+        const Work wk = a.ptiles[w];
+        if (a.steps_left[wk.scene] == 0) continue;
+        const SceneDev S = a.scenes[wk.scene];  // by value: the list stores cannot alias it
+        if ((S.flags & kFlagOrdered) != 0) continue;
+        const int p = wk.start + (int)threadIdx.x;
+        const bool valid = p < S.p_off + S.n;
+        const float4 xi = a.spos[valid ? p : S.p_off];
+        const float4* sp = a.spos + S.p_off;
+        uint32_t* col = &buf[threadIdx.x >> 5][0][threadIdx.x & 31];
+        ListOut out = {a.nlist + (size_t)wk.start * kNbCap + 4 * threadIdx.x, 4 * blockDim.x, col, col, 0};
+        float rho = 0.0f;
+        const f2 nzero = neg_zero();
+        auto row = [&](uint32_t st, uint32_t en) {
+            density_row<FM>(S, sp, -xi.x, -xi.y, -xi.z, nzero, st, en, out, rho);
+        };
+        if (S.reach == 1)
+            for_rows_ahead<1>(a, S, xi, valid, row);
+        else if (S.reach == 2)
+            for_rows_ahead<2>(a, S, xi, valid, row);
+        else
+            for_rows_any(a, S, xi, valid, row);
+        const int cnt = out.finish();
+        if (!valid) continue;
+        if (!FM) rho = density_sum_exact(a, S, xi, out.nl, out.stride, cnt, nzero);
+        a.ncnt[p] = cnt;
+        const float P = fm(S.k, fs(rho, S.p0));
+        const float Ai = fdv(P, fm(rho, rho)), Bi = fdv(S.mass, rho);
+        a.dyn[p] = make_float4(rho, Ai, Bi, P);
+        if (pack) {
             const float4 vi = a.svel[p];
             a.fdat[2 * (size_t)p] = make_float4(xi.x, xi.y, xi.z, Ai);
             a.fdat[2 * (size_t)p + 1] = make_float4(vi.x, vi.y, vi.z, Bi);
@@ -1024,19 +1243,17 @@ __global__ void __launch_bounds__(kMaxTile, MINB) k_force(DevArrays a) {
                     if (dist2(fs(xi.x, xj.x), fs(xi.y, xj.y), fs(xi.z, xj.z)) <= S.smax) pair(j, xj);
                 });
             } else {
-                const uint32_t* nl = a.nlist + (size_t)wk.start * kNbCap + li;
-                const int stride = lstride;
-                uint32_t j0 = cnt > 0 ? __ldg(nl) : 0u;
-                uint32_t j1 = cnt > 1 ? __ldg(nl + stride) : 0u;
+                const uint32_t* nl = a.nlist + (size_t)wk.start * kNbCap;
+                auto entry = [&](int q) { return q < cnt ? __ldg(nl + list_at(q, li, lstride)) : 0u; };
+                uint32_t j0 = entry(0), j1 = entry(1);
                 float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), v0 = x0, d0 = x0;
                 if (cnt > 0) {
                     x0 = __ldg(sp + j0);
                     v0 = __ldg(sv + j0);
                     d0 = __ldg(sd + j0);
                 }
-                nl += 2 * stride;
-                for (int q = 0; q < cnt; ++q, nl += stride) {
-                    const uint32_t j2 = (q + 2 < cnt) ? __ldg(nl) : 0u;
+                for (int q = 0; q < cnt; ++q) {
+                    const uint32_t j2 = entry(q + 2);
                     float4 x1 = x0, v1 = v0, d1 = d0;
                     if (q + 1 < cnt) {
                         x1 = __ldg(sp + j1);
@@ -1074,6 +1291,7 @@ struct PairIn {
 
 struct PairConst {
     float h, hh, hh3, cg, cs, mass, clamp;
+    f2 nzero;
 };
 
 template <bool FM>
@@ -1114,9 +1332,9 @@ __device__ __forceinline__ void force_two(const PairConst& K, ForceAcc& acc, con
         const float la = fsq(a.s), lb = fsq(b.s);
         const f2 cg = pk(K.cg);
         const f2 L = pk(la, lb);
-        const f2 hs = fma2(mulr2(L, L), pk(-1.0f), pk(K.hh));
-        const f2 lap = mul2(mul2(cg, hs), fma2(mulr2(mul2(pk(7.0f), L), L), pk(-1.0f), pk(K.hh3)));
-        const f2 lB = mulr2(pk(-a.B, -lapB), lap);
+        const f2 hs = fma2(mulr2(L, L, K.nzero), pk(-1.0f), pk(K.hh));
+        const f2 lap = mul2(mul2(cg, hs), fma2(mulr2(mul2(pk(7.0f), L), L, K.nzero), pk(-1.0f), pk(K.hh3)));
+        const f2 lB = mulr2(pk(-a.B, -lapB), lap, K.nzero);
         acc.cfl = fa(acc.cfl, lo(lB));
         acc.cfl = fa(acc.cfl, hi(lB));
         const f2 inv = pk(__frcp_rn(fmaxf(la, K.clamp)), __frcp_rn(fmaxf(lb, K.clamp)));
@@ -1127,21 +1345,21 @@ __device__ __forceinline__ void force_two(const PairConst& K, ForceAcc& acc, con
         const f2 lv = mul2(cs, d);
         const f2 pw = mul2(hs, hs);
         const f2 x = pk(a.x, b.x), y = pk(a.y, b.y), z = pk(a.z, b.z);
-        const f2 gx = mulr2(coef, mul2(mul2(mul2(x, inv), cs), pw2));
-        const f2 gy = mulr2(coef, mul2(mul2(mul2(y, inv), cs), pw2));
-        const f2 gz = mulr2(coef, mul2(mul2(mul2(z, inv), cs), pw2));
+        const f2 gx = mulr2(coef, mul2(mul2(mul2(x, inv), cs), pw2), K.nzero);
+        const f2 gy = mulr2(coef, mul2(mul2(mul2(y, inv), cs), pw2), K.nzero);
+        const f2 gz = mulr2(coef, mul2(mul2(mul2(z, inv), cs), pw2), K.nzero);
         acc.fpx = fa(fa(acc.fpx, lo(gx)), hi(gx));
         acc.fpy = fa(fa(acc.fpy, lo(gy)), hi(gy));
         acc.fpz = fa(fa(acc.fpz, lo(gz)), hi(gz));
-        const f2 vx = mulr2(mul2(pk(a.vx, b.vx), B), lv);
-        const f2 vy = mulr2(mul2(pk(a.vy, b.vy), B), lv);
-        const f2 vz = mulr2(mul2(pk(a.vz, b.vz), B), lv);
+        const f2 vx = mulr2(mul2(pk(a.vx, b.vx), B), lv, K.nzero);
+        const f2 vy = mulr2(mul2(pk(a.vy, b.vy), B), lv, K.nzero);
+        const f2 vz = mulr2(mul2(pk(a.vz, b.vz), B), lv, K.nzero);
         acc.fvx = fa(fa(acc.fvx, lo(vx)), hi(vx));
         acc.fvy = fa(fa(acc.fvy, lo(vy)), hi(vy));
         acc.fvz = fa(fa(acc.fvz, lo(vz)), hi(vz));
-        const f2 nx = mulr2(B, mul2(mul2(x, cg), pw));
-        const f2 ny = mulr2(B, mul2(mul2(y, cg), pw));
-        const f2 nz = mulr2(B, mul2(mul2(z, cg), pw));
+        const f2 nx = mulr2(B, mul2(mul2(x, cg), pw), K.nzero);
+        const f2 ny = mulr2(B, mul2(mul2(y, cg), pw), K.nzero);
+        const f2 nz = mulr2(B, mul2(mul2(z, cg), pw), K.nzero);
         acc.nx = fa(fa(acc.nx, lo(nx)), hi(nx));
         acc.ny = fa(fa(acc.ny, lo(ny)), hi(ny));
         acc.nz = fa(fa(acc.nz, lo(nz)), hi(nz));
@@ -1228,10 +1446,10 @@ __global__ void __launch_bounds__(kMaxTile, FM ? 3 : 4) k_force_rec(const __grid
         const int cnt = a.ncnt[p];
         if (cnt <= kNbCap) {
             const float4* fd = a.fdat + 2 * (size_t)S.p_off;
-            const uint32_t* nl = a.nlist + (size_t)wk.start * kNbCap + li;
-            const int stride = a.tile;
+            const uint32_t* nl = a.nlist + (size_t)wk.start * kNbCap + 4 * li;
+            const uint32_t stride = 4 * a.tile;
             const PairConst K = {S.h, S.hh, FM ? 3.0f * S.hh : fm(fm(3.0f, S.h), S.h), S.c_grad, S.c_spiky, S.mass,
-                                 FM ? S.cthr * S.cthr : S.cthr};
+                                 FM ? S.cthr * S.cthr : S.cthr, neg_zero()};
             // pairs closer than the threshold (with a margin) take the general
             // form, and so do all pairs of a particle whose own velocity or
             // factors are not finite (zero times those is not zero)
@@ -1241,48 +1459,49 @@ __global__ void __launch_bounds__(kMaxTile, FM ? 3 : 4) k_force_rec(const __grid
             const bool odd = !((nvx + nvy + nvz) * 0.0f + (Ai + hi(me.vzB)) * 0.0f == 0.0f);
             const float c2 = odd ? INFINITY : S.cthr * S.cthr * 1.0001f;
             const bool rec = REC && (S.flags & kFlagRecord) != 0;
-            uint32_t j0 = pl, j1 = pl, k0 = pl, k1 = pl;  // past the end: the particle itself
-            if (0 < cnt) j0 = __ldg(nl);
-            if (1 < cnt) j1 = __ldg(nl + stride);
-            if (2 < cnt) k0 = __ldg(nl + 2 * stride);
-            if (3 < cnt) k1 = __ldg(nl + 3 * stride);
-            nl += 4 * stride;
+            // the list, two entries at a time; past its end: the particle itself
+            uint32_t step = 2;  // to the next two: within the group of four, then to the next group
+            auto two_at = [&](int q) {
+                uint2 e = make_uint2(pl, pl);
+                if (q < cnt) e = __ldg(reinterpret_cast<const uint2*>(nl));
+                if (q + 1 >= cnt) e.y = pl;
+                nl += step;
+                step = stride - step;
+                return e;
+            };
+            uint2 j = two_at(0), k = two_at(2);
             Rec ra, rb;
             if (FM) {
-                ra = ld_rec(fd + 2 * j0);
-                rb = ld_rec(fd + 2 * j1);
+                ra = ld_rec(fd + 2 * j.x);
+                rb = ld_rec(fd + 2 * j.y);
             }
             for (int q = 0; q < cnt; q += 2) {
                 if (!FM) {
-                    ra = ld_rec(fd + 2 * j0);
-                    rb = ld_rec(fd + 2 * j1);
+                    ra = ld_rec(fd + 2 * j.x);
+                    rb = ld_rec(fd + 2 * j.y);
                 }
                 const PairIn A = pair_in<FM>(ra, nxi, nyi, nzi, Ai, nvx, nvy, nvz);
                 const PairIn B = pair_in<FM>(rb, nxi, nyi, nzi, Ai, nvx, nvy, nvz);
                 if (FM) {
-                    ra = ld_rec(fd + 2 * k0);
-                    rb = ld_rec(fd + 2 * k1);
+                    ra = ld_rec(fd + 2 * k.x);
+                    rb = ld_rec(fd + 2 * k.y);
                 }
                 bool general = false;
-                if (fminf(A.s, B.s) < c2) general = odd || (A.s < c2 && j0 != pl) || (B.s < c2 && j1 != pl);
+                if (fminf(A.s, B.s) < c2) general = odd || (A.s < c2 && j.x != pl) || (B.s < c2 && j.y != pl);
                 if (REC && rec) {
                     const float4* sp = a.spos + S.p_off;
-                    if (j0 != pl) acc.nb = max(acc.nb, __float_as_int(__ldg(&sp[j0].w))), acc.any = 1;
-                    if (j1 != pl) acc.nb = max(acc.nb, __float_as_int(__ldg(&sp[j1].w))), acc.any = 1;
+                    if (j.x != pl) acc.nb = max(acc.nb, __float_as_int(__ldg(&sp[j.x].w))), acc.any = 1;
+                    if (j.y != pl) acc.nb = max(acc.nb, __float_as_int(__ldg(&sp[j.y].w))), acc.any = 1;
                 }
                 const bool two = q + 1 < cnt;
                 if (!general) {
                     force_two<FM>(K, acc, A, B, two ? B.B : 0.0f);
                 } else {
-                    force_one<FM>(S, acc, A, j0 == pl);
-                    if (two) force_one<FM>(S, acc, B, j1 == pl);
+                    force_one<FM>(S, acc, A, j.x == pl);
+                    if (two) force_one<FM>(S, acc, B, j.y == pl);
                 }
-                j0 = k0;
-                j1 = k1;
-                k0 = k1 = pl;
-                if (q + 4 < cnt) k0 = __ldg(nl);
-                if (q + 5 < cnt) k1 = __ldg(nl + stride);
-                nl += 2 * stride;
+                j = k;
+                k = two_at(q + 4);
             }
         }
         const float4 xi = a.spos[p];
@@ -1657,7 +1876,7 @@ __device__ __forceinline__ void density_group_particle(const DevArrays& a, const
             const unsigned b = (__ballot_sync(g.mask, in) & g.mask) >> g.gbase;
             const int at = cnt + __popc(b & below);
             if (in) {
-                if (nl && at < kNbCap) nl[(size_t)at * stride] = j;
+                if (nl && at < kNbCap) nl[(size_t)(at >> 2) * stride + (at & 3)] = j;
                 term[at - done] = s;
             }
             cnt += __popc(b);
@@ -1694,8 +1913,8 @@ __global__ void __launch_bounds__(256, 5) k_density_group(const __grid_constant_
     if (p >= 0) {
         int* soff = s_off + (threadIdx.x & ~(G - 1));
         float* term = s_term[wid];
-        const int stride = lane_lists ? a.tile : 1;
-        uint32_t* nl = a.nlist ? a.nlist + (lane_lists ? (size_t)wk.start * kNbCap + l : (size_t)p * kNbCap) : nullptr;
+        const int stride = 4 * (lane_lists ? a.tile : 1);
+        uint32_t* nl = a.nlist ? a.nlist + (lane_lists ? (size_t)wk.start * kNbCap + 4 * l : (size_t)p * kNbCap) : nullptr;
         int cnt, left;
         float part;
         if (S.reach == 1)
@@ -1968,10 +2187,10 @@ __global__ void __launch_bounds__(kMaxTile + 32, MINB) k_force_tma(DevArrays a, 
                     ok = false;
                     break;
                 }
-                const uint32_t* e = nl + (size_t)q * T + per * lane;
                 uint4 jj[2];
                 for (int g = 0; g < per; g += 4) {
-                    jj[g / 4] = *reinterpret_cast<const uint4*>(e + g);
+                    const uint32_t* e = nl + list_at(q, per * lane + g, T);
+                    jj[g / 4] = make_uint4(e[0], e[4], e[8], e[12]);
                     *reinterpret_cast<uint4*>(jring + (size_t)st * T + per * lane + g) = jj[g / 4];
                 }
                 __syncwarp();
@@ -2266,37 +2485,6 @@ static size_t list_bytes(const LaunchShape& s) { return (size_t)kListCap * s.til
 // budget alone (4 resident blocks of 256 threads); bit 6 pairs the density pass's
 // candidate loads; bit 7 with bit 3 packs each particle's force-pass inputs
 // into one 32-byte record.
-template <int MINB, bool DYN, bool FM>
-static void launch_density_nl_d(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    const bool x2 = (s.variant & 64) != 0, pack = s.pack;
-    const int grid = DYN ? s.grid_dyn : s.grid_p;
-    if (x2 && pack)
-        k_density<false, false, MINB, true, true, true, DYN, FM><<<grid, s.tile, 0, st>>>(a);
-    else if (x2)
-        k_density<false, false, MINB, true, true, false, DYN, FM><<<grid, s.tile, 0, st>>>(a);
-    else if (pack)
-        k_density<false, false, MINB, true, false, true, DYN, FM><<<grid, s.tile, 0, st>>>(a);
-    else
-        k_density<false, false, MINB, true, false, false, DYN, FM><<<grid, s.tile, 0, st>>>(a);
-}
-
-// Bit 16 (65536): the list-writing density pass takes its work in warp
-// slices from a counter (dynamic scheduling; same bits).  Bit 17 (131072):
-// fast arithmetic (density_term_fast; not the same bits).
-template <int MINB>
-static void launch_density_nl(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    const bool fm = (s.variant & 131072) != 0;
-    if (s.variant & 65536) {
-        if (fm)
-            launch_density_nl_d<MINB, true, true>(a, s, st);
-        else
-            launch_density_nl_d<MINB, true, false>(a, s, st);
-    } else if (fm)
-        launch_density_nl_d<MINB, false, true>(a, s, st);
-    else
-        launch_density_nl_d<MINB, false, false>(a, s, st);
-}
-
 // Variant bit 8 (with bit 3): the cooperative passes, G lanes per particle.
 // Density: 32 lanes (bit 11: 16).  Force: 8 lanes (bit 9: 4, bit 10: 16).
 // Bit 7 packs the force-pass inputs as in the per-lane passes; bit 2
@@ -2397,12 +2585,10 @@ void launch_density(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     if (s.density_group) {
         launch_density_group(a, s, (s.variant & 131072) != 0, st);
     } else if (s.variant & 8) {
-        if (relaxed)
-            launch_density_nl<4>(a, s, st);
-        else if (s.variant & 32)
-            launch_density_nl<4>(a, s, st);
+        if (s.variant & 131072)
+            k_density_list<true><<<s.grid_p, s.tile, 0, st>>>(a, s.pack);
         else
-            launch_density_nl<8>(a, s, st);
+            k_density_list<false><<<s.grid_p, s.tile, 0, st>>>(a, s.pack);
     } else if (s.variant & 1) {
         if (relaxed)
             k_density<false, true, 4><<<s.grid_p, s.tile, list_bytes(s), st>>>(a);

@@ -42,10 +42,11 @@ struct DevArrays {
     // in-range neighbour lists written by the density pass and read by the
     // force pass (variant bit 3), in traversal order.  Each work tile of T
     // particles starting at sorted index t owns kNbCap * T entries from
-    // t * kNbCap on, slot-major: entry q of the tile's lane l at q * T + l,
-    // so lanes at the same slot touch consecutive words and a tile's list
-    // stays in one compact region.  ncnt[p] = in-range count (may exceed
-    // kNbCap: that particle's force pass then walks the cells).
+    // t * kNbCap on, in groups of four: entry q of the tile's lane l at
+    // ((q / 4) * T + l) * 4 + q % 4, so a lane writes 16 bytes at a time, next
+    // to its neighbour lanes' (passes that take a group of lanes per particle
+    // keep each particle's entries together instead).  ncnt[p] = in-range
+    // count (may exceed kNbCap: that particle's force pass then walks the cells).
     uint32_t* nlist;
     int32_t* ncnt;
     // packed neighbour records, two float4 per sorted particle:
