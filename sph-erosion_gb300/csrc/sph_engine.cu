@@ -1249,7 +1249,7 @@ void System::enqueue_step(const DevArrays& a, const LaunchShape& s, cudaEvent_t*
         Range r("sph/terrain");
         if (any_terrain_ && s.grid_t > 0) launch_terrain(a, s, st_);
         mark(7);
-        if (any_limited_) launch_tick(a, (int)scenes_.size(), st_);
+        if (any_limited_) launch_tick(a, s, (int)scenes_.size(), st_);
         mark(8);
     }
 }

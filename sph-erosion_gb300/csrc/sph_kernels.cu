@@ -29,6 +29,17 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 
+// The kernels of a step follow one another on one stream and each needs all of
+// the one before.  In small systems they are launched with programmatic
+// serialization (launch): a kernel's blocks may then come to the SMs once all
+// of the previous kernel's have started, and wait here until it has completed
+// and its writes are visible.  Every thread of every kernel of the step calls
+// this first: a kernel that has completed implies that all before it have.
+__device__ __forceinline__ void step_enter() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fs(float a, float b) { return __fsub_rn(a, b); }
@@ -575,6 +586,7 @@ __device__ __forceinline__ Run run_of(uint32_t v, unsigned mask, int lane) {
 constexpr int kKeyTiles = 4;
 
 __global__ void __launch_bounds__(kMaxTile) k_keys(DevArrays a) {
+    step_enter();
     const int nwork = *a.n_ptiles;
     const int lane = threadIdx.x & 31;
     for (int w0 = blockIdx.x * kKeyTiles; w0 < nwork; w0 += gridDim.x * kKeyTiles) {
@@ -664,6 +676,7 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* sh) {
 // chunk totals of its scene, so no block waits on another.  Counts are
 // cleared for the next step.
 __global__ void __launch_bounds__(kScanThreads) k_scan(DevArrays a) {
+    step_enter();
     __shared__ uint32_t sh[kScanThreads / 32];
     const int nwork = *a.n_ctiles;
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
@@ -706,6 +719,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(DevArrays a) {
 // scatter: place each particle's index at its cell's offset + slot, and clear
 // the chunk totals (the scan that read them has finished).
 __global__ void __launch_bounds__(kMaxTile) k_scatter(DevArrays a) {
+    step_enter();
     const int nwork = *a.n_ptiles;
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
         const Work wk = a.ptiles[w];
@@ -730,6 +744,7 @@ __global__ void __launch_bounds__(kMaxTile) k_scatter(DevArrays a) {
 // so results never depend on atomic arrival order) and gather the state into
 // the sorted arrays.
 __global__ void __launch_bounds__(kMaxTile) k_reorder(DevArrays a) {
+    step_enter();
     const int nwork = *a.n_ptiles;
     if (a.ctr && blockIdx.x == 0 && threadIdx.x < 2) a.ctr[threadIdx.x] = 0u;  // for this step's neighbour kernels
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
@@ -792,6 +807,7 @@ __device__ __forceinline__ int first_slice(unsigned* ctr) {
 // neighbour density, so the autotuner picks it.
 template <bool ORDERED, bool LISTED, int MINB>
 __global__ void __launch_bounds__(kMaxTile, MINB) k_density(DevArrays a) {
+    step_enter();
     extern __shared__ uint32_t list[];
     const int nwork = *a.n_ptiles;
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
@@ -1052,6 +1068,7 @@ __device__ __forceinline__ float density_sum_exact(const DevArrays& a, const Sce
 // 318 us; exact, cells of h, 488 -> 444 us.
 template <bool FM>
 __global__ void __launch_bounds__(kMaxTile, 3) k_density_list(const __grid_constant__ DevArrays a, bool pack) {
+    step_enter();
     __shared__ uint32_t buf[kMaxTile / 32][kBuf][32];
     const int nwork = *a.n_ptiles;
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
@@ -1195,6 +1212,7 @@ __device__ __forceinline__ void integrate_and_store(const DevArrays& a, const Sc
 // systems whose HBM budget has no room for the packed records (k_force_rec).
 template <bool ORDERED, int MINB, bool NL = false, bool DYN = false, bool FM = false>
 __global__ void __launch_bounds__(kMaxTile, MINB) k_force(DevArrays a) {
+    step_enter();
     extern __shared__ uint32_t list[];
     const int nwork = *a.n_ptiles;
     const int spt = DYN ? a.tile / 32 : 1;  // slices per tile
@@ -1430,6 +1448,7 @@ __device__ __noinline__ void force_cells(const DevArrays& a, const SceneDev& S, 
 // faster with 32 warps and no records in flight (364 vs 375 us).
 template <bool FM, bool REC>
 __global__ void __launch_bounds__(kMaxTile, FM ? 3 : 4) k_force_rec(const __grid_constant__ DevArrays a) {
+    step_enter();
     const int nwork = *a.n_ptiles;
     const int spt = a.tile / 32;
     for (int sl = first_slice<true>(a.ctr + 1); sl < nwork * spt; sl = next_slice<true>(a.ctr + 1, sl)) {
@@ -1673,6 +1692,7 @@ __device__ __forceinline__ void density_coop_particle(const DevArrays& a, const 
 
 template <int G, bool PACK>
 __global__ void __launch_bounds__(256) k_density_coop(DevArrays a) {
+    step_enter();
     __shared__ int s_off[256];
     const Group<G> g;
     int* soff = s_off + (threadIdx.x & ~(G - 1));
@@ -1703,6 +1723,7 @@ __global__ void __launch_bounds__(256) k_density_coop(DevArrays a) {
 // overflowed has the group split its cell rows instead (row r to lane r mod G).
 template <int G, bool PACK, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_force_coop(DevArrays a) {
+    step_enter();
     const Group<G> g;
     const int group = threadIdx.x / G, ngroups = blockDim.x / G;
     const int nwork = *a.n_ptiles;
@@ -1895,6 +1916,7 @@ __device__ __forceinline__ void density_group_particle(const DevArrays& a, const
 template <bool FM>
 __global__ void __launch_bounds__(256, 5) k_density_group(const __grid_constant__ DevArrays a, bool lane_lists,
                                                           bool pack) {
+    step_enter();
     constexpr int G = 32, N = 256 / G;
     __shared__ int s_off[256];
     __shared__ float s_term[N][kTerms + 1];
@@ -1993,6 +2015,7 @@ __device__ __forceinline__ void pair_values(const SceneDev& S, float rx, float r
 
 template <bool FM, bool REC>
 __global__ void __launch_bounds__(256, 4) k_force_group(const __grid_constant__ DevArrays a) {
+    step_enter();
     constexpr int G = 16, N = 256 / G, V = kPairValues<FM>, W = G + 1;
     __shared__ float s_val[N][V][W];
     __shared__ float s_sum[N][13];  // the ten sums, NeighbId, whether there is a neighbour; the particle
@@ -2139,6 +2162,7 @@ __device__ __forceinline__ void tma_gather4(void* dst, const CUtensorMap* map, i
 
 template <int MINB>
 __global__ void __launch_bounds__(kMaxTile + 32, MINB) k_force_tma(DevArrays a, const __grid_constant__ CUtensorMap fmap) {
+    step_enter();
     extern __shared__ unsigned char smem_raw[];
     __shared__ int s_m;
     const int T = (int)blockDim.x - 32;  // consumers: 128 or 256
@@ -2260,6 +2284,7 @@ size_t force_tma_smem(int tile) {
 // with 16-byte loads and stores (a scene's vertices start on a 512-vertex
 // boundary, so every thread's first vertex is 4-aligned).
 __global__ void __launch_bounds__(kMaxTile / 4) k_terrain(DevArrays a) {
+    step_enter();
     const int nwork = *a.n_ttiles;
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
         const Work wk = a.ttiles[w];
@@ -2282,6 +2307,7 @@ __global__ void __launch_bounds__(kMaxTile / 4) k_terrain(DevArrays a) {
 }
 
 __global__ void k_tick(int* steps_left, int nscenes) {
+    step_enter();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < nscenes && steps_left[s] > 0) steps_left[s] -= 1;
 }
@@ -2381,19 +2407,41 @@ __global__ void __launch_bounds__(256) k_diag(DevArrays a, double* partial, long
     }
 }
 
+// Launch of a kernel of the step (step_enter); early: with programmatic
+// serialization.  It hides a kernel's launch behind the one before it: of
+// 18,432 particles or less a step takes 12 us less launched by itself and 1 to
+// 3 in a graph.  In large systems blocks that wait cost more than that (a step,
+// us, with and without: 100,000 particles 127 vs 113, 1,048,576 862 vs 818,
+// 8.4M 5,367 vs 4,949): the list passes keep the L1 split of the kernel they
+// overlapped.
+template <class... P, class... A>
+void launch(bool early, void (*k)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)block);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = early ? 1 : 0;
+    cudaLaunchKernelEx(&c, k, P(args)...);
+}
+
 }  // namespace
 
 void launch_keys(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    k_keys<<<(s.grid_p + kKeyTiles - 1) / kKeyTiles, s.tile, 0, st>>>(a);
+    launch(s.early, k_keys, (s.grid_p + kKeyTiles - 1) / kKeyTiles, s.tile, 0, st, a);
 }
 void launch_scan(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    k_scan<<<s.grid_c, kScanThreads, 0, st>>>(a);
+    launch(s.early, k_scan, s.grid_c, kScanThreads, 0, st, a);
 }
 void launch_scatter(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    k_scatter<<<s.grid_p, s.tile, 0, st>>>(a);
+    launch(s.early, k_scatter, s.grid_p, s.tile, 0, st, a);
 }
 void launch_reorder(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    k_reorder<<<s.grid_p, s.tile, 0, st>>>(a);
+    launch(s.early, k_reorder, s.grid_p, s.tile, 0, st, a);
 }
 namespace {
 // Traversal counters of one scene: [rows visited, candidates tested,
@@ -2493,14 +2541,14 @@ static void launch_density_coop(const DevArrays& a, const LaunchShape& s, cudaSt
     const bool pack = (s.variant & 128) != 0;
     if (s.variant & 2048) {
         if (pack)
-            k_density_coop<16, true><<<s.grid_p, s.tile, 0, st>>>(a);
+            launch(s.early, k_density_coop<16, true>, s.grid_p, s.tile, 0, st, a);
         else
-            k_density_coop<16, false><<<s.grid_p, s.tile, 0, st>>>(a);
+            launch(s.early, k_density_coop<16, false>, s.grid_p, s.tile, 0, st, a);
     } else {
         if (pack)
-            k_density_coop<32, true><<<s.grid_p, s.tile, 0, st>>>(a);
+            launch(s.early, k_density_coop<32, true>, s.grid_p, s.tile, 0, st, a);
         else
-            k_density_coop<32, false><<<s.grid_p, s.tile, 0, st>>>(a);
+            launch(s.early, k_density_coop<32, false>, s.grid_p, s.tile, 0, st, a);
     }
 }
 
@@ -2510,19 +2558,19 @@ static void launch_force_coop_b(const DevArrays& a, const LaunchShape& s, cudaSt
     const int gsel = (s.variant >> 9) & 3;
     if (gsel == 1) {
         if (pack)
-            k_force_coop<4, true, MINB><<<s.grid_p, s.tile, 0, st>>>(a);
+            launch(s.early, k_force_coop<4, true, MINB>, s.grid_p, s.tile, 0, st, a);
         else
-            k_force_coop<4, false, MINB><<<s.grid_p, s.tile, 0, st>>>(a);
+            launch(s.early, k_force_coop<4, false, MINB>, s.grid_p, s.tile, 0, st, a);
     } else if (gsel == 2) {
         if (pack)
-            k_force_coop<16, true, MINB><<<s.grid_p, s.tile, 0, st>>>(a);
+            launch(s.early, k_force_coop<16, true, MINB>, s.grid_p, s.tile, 0, st, a);
         else
-            k_force_coop<16, false, MINB><<<s.grid_p, s.tile, 0, st>>>(a);
+            launch(s.early, k_force_coop<16, false, MINB>, s.grid_p, s.tile, 0, st, a);
     } else {
         if (pack)
-            k_force_coop<8, true, MINB><<<s.grid_p, s.tile, 0, st>>>(a);
+            launch(s.early, k_force_coop<8, true, MINB>, s.grid_p, s.tile, 0, st, a);
         else
-            k_force_coop<8, false, MINB><<<s.grid_p, s.tile, 0, st>>>(a);
+            launch(s.early, k_force_coop<8, false, MINB>, s.grid_p, s.tile, 0, st, a);
     }
 }
 
@@ -2539,22 +2587,22 @@ static void launch_density_group(const DevArrays& a, const LaunchShape& s, bool 
     const int blocks = s.grid_p * s.tile / 8;
     const bool lane_lists = !s.force_group, pack = lane_lists && s.pack;
     if (fast)
-        k_density_group<true><<<blocks, 256, 0, st>>>(a, lane_lists, pack);
+        launch(s.early, k_density_group<true>, blocks, 256, 0, st, a, lane_lists, pack);
     else
-        k_density_group<false><<<blocks, 256, 0, st>>>(a, lane_lists, pack);
+        launch(s.early, k_density_group<false>, blocks, 256, 0, st, a, lane_lists, pack);
 }
 
 static void launch_force_group(const DevArrays& a, const LaunchShape& s, bool fast, cudaStream_t st) {
     const int blocks = s.grid_p * s.tile / 16;
     if (s.record) {
         if (fast)
-            k_force_group<true, true><<<blocks, 256, 0, st>>>(a);
+            launch(s.early, k_force_group<true, true>, blocks, 256, 0, st, a);
         else
-            k_force_group<false, true><<<blocks, 256, 0, st>>>(a);
+            launch(s.early, k_force_group<false, true>, blocks, 256, 0, st, a);
     } else if (fast)
-        k_force_group<true, false><<<blocks, 256, 0, st>>>(a);
+        launch(s.early, k_force_group<true, false>, blocks, 256, 0, st, a);
     else
-        k_force_group<false, false><<<blocks, 256, 0, st>>>(a);
+        launch(s.early, k_force_group<false, false>, blocks, 256, 0, st, a);
 }
 
 // Which passes of a step take a group of lanes per particle: the per-lane list
@@ -2570,6 +2618,7 @@ static void launch_force_group(const DevArrays& a, const LaunchShape& s, bool fa
 void group_rules(LaunchShape& s) {
     const int64_t n = (int64_t)s.grid_p * s.tile;
     const bool lists = (s.variant & (8 | 256)) == 8;
+    s.early = n <= 18432;
     s.density_group = lists && n <= ((s.variant & 131072) ? 12288 : 18432);
     s.force_group = s.density_group && n <= ((s.variant & (131072 | 16)) == (131072 | 16) ? 8192 : 18432);
 }
@@ -2586,23 +2635,23 @@ void launch_density(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
         launch_density_group(a, s, (s.variant & 131072) != 0, st);
     } else if (s.variant & 8) {
         if (s.variant & 131072)
-            k_density_list<true><<<s.grid_p, s.tile, 0, st>>>(a, s.pack);
+            launch(s.early, k_density_list<true>, s.grid_p, s.tile, 0, st, a, s.pack);
         else
-            k_density_list<false><<<s.grid_p, s.tile, 0, st>>>(a, s.pack);
+            launch(s.early, k_density_list<false>, s.grid_p, s.tile, 0, st, a, s.pack);
     } else if (s.variant & 1) {
         if (relaxed)
-            k_density<false, true, 4><<<s.grid_p, s.tile, list_bytes(s), st>>>(a);
+            launch(s.early, k_density<false, true, 4>, s.grid_p, s.tile, list_bytes(s), st, a);
         else
-            k_density<false, true, 8><<<s.grid_p, s.tile, list_bytes(s), st>>>(a);
+            launch(s.early, k_density<false, true, 8>, s.grid_p, s.tile, list_bytes(s), st, a);
     } else {
         if (relaxed)
-            k_density<false, false, 4><<<s.grid_p, s.tile, 0, st>>>(a);
+            launch(s.early, k_density<false, false, 4>, s.grid_p, s.tile, 0, st, a);
         else
-            k_density<false, false, 8><<<s.grid_p, s.tile, 0, st>>>(a);
+            launch(s.early, k_density<false, false, 8>, s.grid_p, s.tile, 0, st, a);
     }
 }
 void launch_density_ordered(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    k_density<true, false, 1><<<s.grid_p, s.tile, 0, st>>>(a);
+    launch(s.early, k_density<true, false, 1>, s.grid_p, s.tile, 0, st, a);
 }
 void launch_force(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     if (coop(s)) {
@@ -2619,38 +2668,38 @@ void launch_force(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     // slices from a counter.
     if (!s.force_group && (s.variant & 262144) && (s.variant & (131072 | 128 | 24)) == (131072 | 128 | 24) && s.fmap) {
         // bit 18: the TMA gather pipeline (fast arithmetic, packed records)
-        k_force_tma<3><<<s.grid_p, s.tile + 32, force_tma_smem(s.tile), st>>>(a, *static_cast<const CUtensorMap*>(s.fmap));
+        launch(s.early, k_force_tma<3>, s.grid_p, s.tile + 32, force_tma_smem(s.tile), st, a, *static_cast<const CUtensorMap*>(s.fmap));
         return;
     }
     if (s.variant & 8) {
         const bool fast = (s.variant & (131072 | 16)) == (131072 | 16);
         if (!s.pack) {
             if (fast)
-                k_force<false, 4, true, true, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
+                launch(s.early, k_force<false, 4, true, true, true>, s.grid_dyn, s.tile, 0, st, a);
             else
-                k_force<false, 4, true, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
+                launch(s.early, k_force<false, 4, true, true>, s.grid_dyn, s.tile, 0, st, a);
         } else if (s.record) {
             if (fast)
-                k_force_rec<true, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
+                launch(s.early, k_force_rec<true, true>, s.grid_dyn, s.tile, 0, st, a);
             else
-                k_force_rec<false, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
+                launch(s.early, k_force_rec<false, true>, s.grid_dyn, s.tile, 0, st, a);
         } else if (fast)
-            k_force_rec<true, false><<<s.grid_dyn, s.tile, 0, st>>>(a);
+            launch(s.early, k_force_rec<true, false>, s.grid_dyn, s.tile, 0, st, a);
         else
-            k_force_rec<false, false><<<s.grid_dyn, s.tile, 0, st>>>(a);
+            launch(s.early, k_force_rec<false, false>, s.grid_dyn, s.tile, 0, st, a);
     } else if (s.variant & 4)
-        k_force<false, 3><<<s.grid_p, s.tile, list_bytes(s), st>>>(a);
+        launch(s.early, k_force<false, 3>, s.grid_p, s.tile, list_bytes(s), st, a);
     else
-        k_force<false, 4><<<s.grid_p, s.tile, list_bytes(s), st>>>(a);
+        launch(s.early, k_force<false, 4>, s.grid_p, s.tile, list_bytes(s), st, a);
 }
 void launch_force_ordered(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    k_force<true, 1><<<s.grid_p, s.tile, 0, st>>>(a);
+    launch(s.early, k_force<true, 1>, s.grid_p, s.tile, 0, st, a);
 }
 void launch_terrain(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    k_terrain<<<s.grid_t, s.tile / 4, 0, st>>>(a);
+    launch(s.early, k_terrain, s.grid_t, s.tile / 4, 0, st, a);
 }
-void launch_tick(const DevArrays& a, int nscenes, cudaStream_t st) {
-    k_tick<<<(nscenes + 127) / 128, 128, 0, st>>>(a.steps_left, nscenes);
+void launch_tick(const DevArrays& a, const LaunchShape& s, int nscenes, cudaStream_t st) {
+    launch(s.early, k_tick, (nscenes + 127) / 128, 128, 0, st, a.steps_left, nscenes);
 }
 void launch_neighbour_counts(const DevArrays& a, const LaunchShape& s, int32_t* out_by_id, cudaStream_t st) {
     k_neighbour_counts<<<s.grid_p, s.tile, 0, st>>>(a, out_by_id);

@@ -73,6 +73,7 @@ struct LaunchShape {
     int grid_t;      // persistent grid of the terrain kernel
     int variant;     // sph_system_config.variant bits (bit 3 only with lists allocated)
     bool pack;       // the density pass writes packed records, the force pass gathers them
+    bool early;      // few particles: each kernel's launch overlaps the kernel before it
     bool density_group, force_group;  // few particles: a group of lanes per particle (group_rules)
     bool record;     // some scene keeps its force records (SPH_FLAG_RECORD)
     int grid_dyn;    // grid of the dynamically scheduled neighbour kernels
@@ -86,14 +87,14 @@ void launch_keys(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_scan(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_scatter(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_reorder(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
-// Sets density_group and force_group from the other members.
+// Sets early, density_group and force_group from the other members.
 void group_rules(LaunchShape& s);
 void launch_density(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_density_ordered(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_force(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_force_ordered(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_terrain(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
-void launch_tick(const DevArrays& a, int nscenes, cudaStream_t st);
+void launch_tick(const DevArrays& a, const LaunchShape& s, int nscenes, cudaStream_t st);
 
 // Inspection and on-demand kernels.
 void launch_neighbour_counts(const DevArrays& a, const LaunchShape& s, int32_t* out_by_id, cudaStream_t st);
