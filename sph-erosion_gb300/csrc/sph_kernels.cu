@@ -1817,11 +1817,14 @@ __global__ void __launch_bounds__(256, MINB) k_force_coop(DevArrays a) {
 // Group number `slot` takes lane slot % T of work tile slot / T.
 constexpr int kTerms = 256;  // density terms a group holds before it adds them
 
-template <int G, int R, bool FM>
-__device__ __forceinline__ void density_group_particle(const DevArrays& a, const SceneDev& S, int p, uint32_t* nl,
-                                                       int stride, int* soff, float* term, const Group<G>& g,
-                                                       int& count, int& left, float& part) {
-    const float4 xi = a.spos[p];
+// The candidate stream of particle p, rows in traversal order, G candidates a
+// window: window(in, j, s, id, b, cnt) receives in every lane of the group its
+// candidate's index, squared distance and id, whether it is in range, the
+// window's in-range lanes and the number in range before it.  Returns the
+// number in range.
+template <int G, int R, class F>
+__device__ __forceinline__ int group_walk(const DevArrays& a, const SceneDev& S, float4 xi, int* soff, const Group<G>& g,
+                                          F&& window) {
     const Probe q = probe_of(S, xi);
     constexpr int XS = R == 1 ? 2 : 1;  // the scene's xsub at this reach
     constexpr int RX = (R > 0 ? R : 1) * XS;
@@ -1841,24 +1844,7 @@ __device__ __forceinline__ void density_group_particle(const DevArrays& a, const
     const float4* sp = a.spos + S.p_off;
     const int side = R > 0 ? 2 * R + 1 : 2 * S.reach + 1;
     const int nrows = side * side;
-    const float mc = S.mass * S.c_poly6;
-    float rho = 0.0f;
-    int cnt = 0, done = 0;  // in-range candidates, terms added
-    auto make_terms = [&]() {  // squared distances to terms
-        __syncwarp(g.mask);
-        for (int k = g.gl; k < cnt - done; k += G) {
-            const float hs = S.hh - term[k];
-            term[k] = FM ? hs * hs * hs : density_term(S, fsq(term[k]));
-        }
-    };
-    auto add_terms = [&]() {
-        make_terms();
-        __syncwarp(g.mask);
-        for (int k = 0; k < cnt - done; ++k) rho = FM ? fmaf(mc, term[k], rho) : fa(rho, term[k]);
-        done = cnt;
-        __syncwarp(g.mask);
-    };
-    const unsigned below = (1u << g.gl) - 1u;
+    int cnt = 0;
     for (int rb = 0; rb < nrows; rb += G) {
         uint32_t st = 0, en = 0;
         if (rb + g.gl < nrows) stencil_row<R>(a, S, q, gx2, rb + g.gl, st, en);
@@ -1887,23 +1873,61 @@ __device__ __forceinline__ void density_group_particle(const DevArrays& a, const
             bool in = false;
             uint32_t j = 0;
             float s = 0.0f;
+            int id = 0;
             if (t < total) {
                 j = (uint32_t)(t + off);
                 const float4 xj = __ldg(sp + j);
                 s = dist2(fs(xi.x, xj.x), fs(xi.y, xj.y), fs(xi.z, xj.z));
                 in = s <= S.smax;
+                id = __float_as_int(xj.w);
             }
-            if (cnt - done > kTerms - G) add_terms();
             const unsigned b = (__ballot_sync(g.mask, in) & g.mask) >> g.gbase;
-            const int at = cnt + __popc(b & below);
-            if (in) {
-                if (nl && at < kNbCap) nl[(size_t)(at >> 2) * stride + (at & 3)] = j;
-                term[at - done] = s;
-            }
+            window(in, j, s, id, b, cnt);
             cnt += __popc(b);
         }
     }
-    make_terms();
+    return cnt;
+}
+
+// The walk for the scene's reach.
+template <int G, class F>
+__device__ __forceinline__ int group_walk_any(const DevArrays& a, const SceneDev& S, float4 xi, int* soff,
+                                              const Group<G>& g, F&& window) {
+    if (S.reach == 1) return group_walk<G, 1>(a, S, xi, soff, g, window);
+    if (S.reach == 2) return group_walk<G, 2>(a, S, xi, soff, g, window);
+    return group_walk<G, 0>(a, S, xi, soff, g, window);
+}
+
+template <int G, int R, bool FM>
+__device__ __forceinline__ void density_group_particle(const DevArrays& a, const SceneDev& S, int p, uint32_t* nl,
+                                                       int stride, int* soff, float* term, const Group<G>& g,
+                                                       int& count, int& left, float& part) {
+    const float mc = S.mass * S.c_poly6;
+    float rho = 0.0f;
+    int done = 0;  // terms added
+    auto make_terms = [&](int cnt) {  // squared distances to terms
+        __syncwarp(g.mask);
+        for (int k = g.gl; k < cnt - done; k += G) {
+            const float hs = S.hh - term[k];
+            term[k] = FM ? hs * hs * hs : density_term(S, fsq(term[k]));
+        }
+    };
+    const unsigned below = (1u << g.gl) - 1u;
+    const int cnt = group_walk<G, R>(a, S, a.spos[p], soff, g, [&](bool in, uint32_t j, float s, int, unsigned b, int n) {
+        if (n - done > kTerms - G) {
+            make_terms(n);
+            __syncwarp(g.mask);
+            for (int k = 0; k < n - done; ++k) rho = FM ? fmaf(mc, term[k], rho) : fa(rho, term[k]);
+            done = n;
+            __syncwarp(g.mask);
+        }
+        if (in) {
+            const int at = n + __popc(b & below);
+            if (nl && at < kNbCap) nl[(size_t)(at >> 2) * stride + (at & 3)] = j;
+            term[at - done] = s;
+        }
+    });
+    make_terms(cnt);
     count = cnt;
     left = cnt - done;
     part = rho;
@@ -2095,6 +2119,146 @@ __global__ void __launch_bounds__(256, 4) k_force_group(const __grid_constant__ 
     __syncthreads();
     if (threadIdx.x >= N) return;
     sum = s_sum[threadIdx.x];
+    p = __float_as_int(sum[12]);
+    if (p < 0) return;
+    const ForceAcc acc = {sum[0], sum[1], sum[2], sum[3], sum[4], sum[5], sum[6], sum[7], sum[8], sum[9],
+                          __float_as_int(sum[10]), __float_as_int(sum[11])};
+    integrate_and_store(a, S, p, a.spos[p], a.svel[p], a.dyn[p].x, acc, true);
+}
+
+// Ordered (validation) passes, a warp per particle: the in-range candidates of
+// the walk are ranked by id, every lane counting the smaller ids of up to four
+// of them, and the terms then added in rank order, which is the reference's
+// order of summation (j ascending).  One lane per particle, sorting its list
+// by insertion in local memory, takes 59 + 67 us for 5,000 particles; these 16 +
+// 18 (group_rules).
+struct OrderedList {
+    uint32_t j[kMaxNb];
+    int id[kMaxNb];
+    float s[kMaxNb];
+};
+
+// Collects and ranks: lane gl's candidates gl, gl + 32, ... have the ranks
+// rank[0], rank[1], ...  Returns the number in the list; more in range than it
+// holds sets the status bit.
+__device__ __forceinline__ int ordered_collect(const DevArrays& a, const SceneDev& S, float4 xi, int* soff,
+                                               OrderedList& l, const Group<32>& g, int* rank) {
+    const unsigned below = (1u << g.gl) - 1u;
+    const int cnt = group_walk_any<32>(a, S, xi, soff, g, [&](bool in, uint32_t j, float s, int id, unsigned b, int n) {
+        const int at = n + __popc(b & below);
+        if (in && at < kMaxNb) l.j[at] = j, l.id[at] = id, l.s[at] = s;
+    });
+    const int m = min(cnt, kMaxNb);
+    if (cnt > kMaxNb && g.gl == 0) atomicOr(a.status, 1u);
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < kMaxNb / 32; ++u) {
+        const int k = g.gl + 32 * u;
+        rank[u] = 0;
+        if (k < m) {
+            const int id = l.id[k];
+            for (int q = 0; q < m; ++q) rank[u] += l.id[q] < id || (l.id[q] == id && l.j[q] < l.j[k]) ? 1 : 0;
+        }
+    }
+    return m;
+}
+
+// The particle of warp `wid` of a block of 8 in tile order; -1: none.
+__device__ __forceinline__ int ordered_particle(const DevArrays& a, int wid, Work& wk) {
+    const int slot = (int)blockIdx.x * 8 + wid, w = slot / a.tile;
+    wk = Work{0, 0};
+    if (w >= *a.n_ptiles) return -1;
+    wk = a.ptiles[w];
+    const SceneDev& S = a.scenes[wk.scene];
+    const int p = wk.start + slot % a.tile;
+    return a.steps_left[wk.scene] != 0 && (S.flags & kFlagOrdered) && p < S.p_off + S.n ? p : -1;
+}
+
+__global__ void __launch_bounds__(256) k_density_ordered(const __grid_constant__ DevArrays a) {
+    step_enter();
+    __shared__ int s_off[8][32];
+    __shared__ OrderedList s_list[8];
+    const Group<32> g;
+    const int wid = threadIdx.x >> 5;
+    Work wk;
+    const int p = ordered_particle(a, wid, wk);
+    if (p < 0) return;
+    const SceneDev& S = a.scenes[wk.scene];
+    OrderedList& l = s_list[wid];
+    int rank[kMaxNb / 32];
+    const int m = ordered_collect(a, S, a.spos[p], s_off[wid], l, g, rank);
+    float t[kMaxNb / 32];
+#pragma unroll
+    for (int u = 0; u < kMaxNb / 32; ++u)
+        if (g.gl + 32 * u < m) t[u] = density_term(S, fsq(l.s[g.gl + 32 * u]));
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < kMaxNb / 32; ++u)
+        if (g.gl + 32 * u < m) l.s[rank[u]] = t[u];
+    __syncwarp();
+    float rho = 0.0f;
+    for (int k = 0; k < m; ++k) rho = fa(rho, l.s[k]);
+    if (g.gl == 0) {
+        const float P = fm(S.k, fs(rho, S.p0));
+        a.dyn[p] = make_float4(rho, fdv(P, fm(rho, rho)), fdv(S.mass, rho), P);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_force_ordered(const __grid_constant__ DevArrays a) {
+    step_enter();
+    constexpr int V = kPairValues<false>;
+    __shared__ int s_off[8][32];
+    __shared__ OrderedList s_list[8];
+    __shared__ float s_val[8][V][33];
+    __shared__ float s_sum[8][13];  // the ten sums, NeighbId, whether there is a neighbour; the particle
+    const Group<32> g;
+    const int wid = threadIdx.x >> 5;
+    Work wk;
+    int p = ordered_particle(a, wid, wk);
+    const SceneDev& S = a.scenes[wk.scene];  // the tile's, the same for the whole block
+    if (p >= 0) {
+        OrderedList& l = s_list[wid];
+        const float4 xi = a.spos[p], vi = a.svel[p];
+        const float Ai = a.dyn[p].y;
+        int rank[kMaxNb / 32];
+        const int m = ordered_collect(a, S, xi, s_off[wid], l, g, rank);
+        uint32_t jr[kMaxNb / 32];
+#pragma unroll
+        for (int u = 0; u < kMaxNb / 32; ++u)
+            if (g.gl + 32 * u < m) jr[u] = l.j[g.gl + 32 * u];
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < kMaxNb / 32; ++u)
+            if (g.gl + 32 * u < m) l.j[rank[u]] = jr[u];
+        __syncwarp();
+        const uint32_t pl = (uint32_t)(p - S.p_off);
+        float acc = 0.0f;
+        int nb = -1, any = 0;
+        for (int b = 0; b < m; b += 32) {
+            if (b + g.gl < m) {
+                const uint32_t j = l.j[b + g.gl];
+                const float4 xj = a.spos[S.p_off + j], vj = a.svel[S.p_off + j], dj = a.dyn[S.p_off + j];
+                if (j != pl) nb = max(nb, __float_as_int(xj.w)), any = 1;
+                float v[V];
+                pair_values<false>(S, fs(xi.x, xj.x), fs(xi.y, xj.y), fs(xi.z, xj.z), fs(vj.x, vi.x), fs(vj.y, vi.y),
+                                   fs(vj.z, vi.z), fa(Ai, dj.y), dj.z, j == pl, v);
+#pragma unroll
+                for (int k = 0; k < V; ++k) s_val[wid][k][g.gl] = v[k];
+            }
+            __syncwarp();
+            if (g.gl < 10)
+                for (int k = 0; k < min(32, m - b); ++k) acc = fa(acc, s_val[wid][g.gl][k]);
+            __syncwarp();
+        }
+        nb = __reduce_max_sync(kFull, nb);
+        any = __reduce_max_sync(kFull, any);
+        if (g.gl < 10) s_sum[wid][g.gl] = acc;
+        if (g.gl == 0) s_sum[wid][10] = __int_as_float(nb), s_sum[wid][11] = __int_as_float(any);
+    }
+    if (g.gl == 0) s_sum[wid][12] = __int_as_float(p);
+    __syncthreads();
+    if (threadIdx.x >= 8) return;
+    const float* sum = s_sum[threadIdx.x];
     p = __float_as_int(sum[12]);
     if (p < 0) return;
     const ForceAcc acc = {sum[0], sum[1], sum[2], sum[3], sum[4], sum[5], sum[6], sum[7], sum[8], sum[9],
@@ -2615,10 +2779,14 @@ static void launch_force_group(const DevArrays& a, const LaunchShape& s, bool fa
 // 27.1; fast, force (beside the group density pass) 8,000 19.1 vs 19.7, 12,000
 // 26.5 vs 24.5.  A system alone on the chip gains up to there from 2.3x (1,000
 // particles: 74 to 32 us) to 1.6x (20,000: 99 to 62 us) a step.
+// The ordered passes' line: density + force, us, a warp per particle vs one lane,
+// 5,000 particles 34 vs 127, 16,384 68 vs 143, 50,000 167 vs 217, 200,000 607 vs
+// 536.
 void group_rules(LaunchShape& s) {
     const int64_t n = (int64_t)s.grid_p * s.tile;
     const bool lists = (s.variant & (8 | 256)) == 8;
     s.early = n <= 18432;
+    s.ordered_group = n <= 32768;
     s.density_group = lists && n <= ((s.variant & 131072) ? 12288 : 18432);
     s.force_group = s.density_group && n <= ((s.variant & (131072 | 16)) == (131072 | 16) ? 8192 : 18432);
 }
@@ -2651,7 +2819,10 @@ void launch_density(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     }
 }
 void launch_density_ordered(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    launch(s.early, k_density<true, false, 1>, s.grid_p, s.tile, 0, st, a);
+    if (s.ordered_group)
+        launch(s.early, k_density_ordered, s.grid_p * s.tile / 8, 256, 0, st, a);
+    else
+        launch(s.early, k_density<true, false, 1>, s.grid_p, s.tile, 0, st, a);
 }
 void launch_force(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     if (coop(s)) {
@@ -2693,7 +2864,10 @@ void launch_force(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
         launch(s.early, k_force<false, 4>, s.grid_p, s.tile, list_bytes(s), st, a);
 }
 void launch_force_ordered(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    launch(s.early, k_force<true, 1>, s.grid_p, s.tile, 0, st, a);
+    if (s.ordered_group)
+        launch(s.early, k_force_ordered, s.grid_p * s.tile / 8, 256, 0, st, a);
+    else
+        launch(s.early, k_force<true, 1>, s.grid_p, s.tile, 0, st, a);
 }
 void launch_terrain(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     launch(s.early, k_terrain, s.grid_t, s.tile / 4, 0, st, a);

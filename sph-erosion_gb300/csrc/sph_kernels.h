@@ -74,7 +74,7 @@ struct LaunchShape {
     int variant;     // sph_system_config.variant bits (bit 3 only with lists allocated)
     bool pack;       // the density pass writes packed records, the force pass gathers them
     bool early;      // few particles: each kernel's launch overlaps the kernel before it
-    bool density_group, force_group;  // few particles: a group of lanes per particle (group_rules)
+    bool density_group, force_group, ordered_group;  // few particles: a group of lanes per particle (group_rules)
     bool record;     // some scene keeps its force records (SPH_FLAG_RECORD)
     int grid_dyn;    // grid of the dynamically scheduled neighbour kernels
     const void* fmap;  // host copy of the CUtensorMap over the packed records (null: none)
@@ -87,7 +87,7 @@ void launch_keys(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_scan(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_scatter(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_reorder(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
-// Sets early, density_group and force_group from the other members.
+// Sets early and the three group members from the others.
 void group_rules(LaunchShape& s);
 void launch_density(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_density_ordered(const DevArrays& a, const LaunchShape& s, cudaStream_t st);

@@ -192,6 +192,7 @@ extern "C" SPH_API int sph_density_static(const sph_params* p, int n, const floa
         s.variant = 0;
         s.pack = false;
         s.early = true;
+        s.ordered_group = false;
         s.density_group = true;  // at most 32,768 particles (group_rules)
         s.force_group = true;    // no list is written
         s.record = false;

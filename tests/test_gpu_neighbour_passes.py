@@ -73,3 +73,32 @@ def test_list_lengths_bit_exact(name, fill, cell_mult):
             assert np.array_equal(got[1], want[1]), (reference, v)
         got = records(name, cell_mult, forms[0], fill, record=False, tile=128)
         assert np.array_equal(got[0][:, :6], want[0][:, :6], equal_nan=True), reference
+
+
+def ordered(sizes, cell_mult, fill):
+    """Records after two ordered steps of clusters, beside `fill` other particles."""
+    rng = np.random.default_rng(7)
+    pos = clusters(rng, sizes)
+    vel = rng.normal(0.0, 0.3, pos.shape).astype(np.float32)
+    pos[5], vel[3, 0] = pos[4], np.inf
+    with S.System(particle_capacity=len(pos) + fill) as sysm:
+        flags = S.SPH_FLAG_RECORD | S.SPH_FLAG_ORDERED
+        prm = dict(REF, box_len=0.9, cell_mult=cell_mult)
+        sc = sysm.scene(S.default_params(**prm, flags=flags), capacity=len(pos))
+        sc.set_particles(pos, vel)
+        if fill:
+            sysm.scene(S.default_params(**prm)).set_particles(np.random.default_rng(1).uniform(-0.8, 0.8, (fill, 3)))
+        sysm.step(2)
+        return sc.get_records()
+
+
+@pytest.mark.parametrize("cell_mult", [1.0, 0.5, 0.3])
+def test_ordered_lists_bit_exact(cell_mult):
+    """A warp per particle (few particles) against one lane per particle; more
+    in-range neighbours than the ordered lists hold (128) are an error in both."""
+    sizes = [k for k in SIZES if k <= 128] + [95, 96, 97]
+    a, b = ordered(sizes, cell_mult, 0), ordered(sizes, cell_mult, 40000)
+    assert np.array_equal(a[0], b[0], equal_nan=True) and np.array_equal(a[1], b[1])
+    for fill in (0, 40000):
+        with pytest.raises(S.SphError):
+            ordered([129, 3], cell_mult, fill)
