@@ -217,6 +217,7 @@ class System {
     int n_ptiles_ = 0, n_ctiles_ = 0, n_ttiles_ = 0;
     bool any_fast_ = false, any_ordered_ = false, any_terrain_ = false, any_limited_ = false,
          any_record_ = false;
+    int64_t max_n_ = 0, max_keys_ = 0;  // largest scene of the work lists
     bool work_dirty_ = true;
 
     cudaGraph_t graph_ = nullptr;

@@ -775,6 +775,76 @@ __global__ void __launch_bounds__(kMaxTile) k_reorder(DevArrays a) {
     }
 }
 
+// The whole sort of a small scene in one block: keys, scan, scatter and reorder
+// with the counts, offsets and order in shared memory.  The four kernels are
+// chains of dependent loads of 5 to 9 us each at these sizes, whatever the
+// number of particles.  Block w takes the scene whose first tile work item w is.
+constexpr int kSortThreads = 1024;
+constexpr int kSortPer = kSmallSort / kSortThreads;  // particles a thread takes
+
+__global__ void __launch_bounds__(kSortThreads) k_sort_small(const __grid_constant__ DevArrays a) {
+    step_enter();
+    extern __shared__ uint32_t sm[];
+    __shared__ uint32_t s_warp[kSortThreads / 32];
+    const int tid = threadIdx.x;
+    if (a.ctr && blockIdx.x == 0 && tid < 2) a.ctr[tid] = 0u;  // for this step's neighbour kernels
+    const Work wk = a.ptiles[blockIdx.x];
+    const SceneDev& S = a.scenes[wk.scene];
+    if (wk.start != S.p_off || a.steps_left[wk.scene] == 0) return;
+    const int n = S.n, nkeys = S.nkeys;
+    const int per = ((nkeys + kSortThreads - 1) / kSortThreads) | 1;  // keys a thread scans; odd: no bank conflicts
+    uint32_t* perm = sm;                 // kSmallSort
+    uint32_t* cnt = sm + kSmallSort;     // per * kSortThreads: counts, then offsets
+    float4 x[kSortPer], v[kSortPer];
+#pragma unroll
+    for (int u = 0; u < kSortPer; ++u) {
+        const int i = tid + u * kSortThreads;
+        if (i < n) x[u] = a.pos[S.p_off + i], v[u] = a.vel[S.p_off + i];
+    }
+    for (int k = tid; k < per * kSortThreads; k += kSortThreads) cnt[k] = 0u;
+    __syncthreads();
+    uint32_t key[kSortPer], slot[kSortPer];
+#pragma unroll
+    for (int u = 0; u < kSortPer; ++u) {
+        const int i = tid + u * kSortThreads;
+        if (i >= n) continue;
+        const Cell c = cell_of(S, x[u].x, x[u].y, x[u].z);
+        key[u] = row_key(a.tab, S, c.cy, c.cz) + (uint32_t)c.cx;
+        a.key[S.p_off + i] = key[u];
+        slot[u] = atomicAdd(cnt + key[u], 1u);
+    }
+    __syncthreads();
+    uint32_t sum = 0;
+    for (int k = 0; k < per; ++k) sum += cnt[tid * per + k];
+    uint32_t run = block_exclusive<kSortThreads>(sum, s_warp);
+    for (int k = 0; k < per; ++k) {
+        const uint32_t c = cnt[tid * per + k];
+        cnt[tid * per + k] = run;
+        run += c;
+    }
+    __syncthreads();
+    for (int k = tid; k < nkeys; k += kSortThreads) a.offsets[S.k_off + k] = cnt[k];
+#pragma unroll
+    for (int u = 0; u < kSortPer; ++u) {
+        const int i = tid + u * kSortThreads;
+        if (i < n) perm[cnt[key[u]] + slot[u]] = (uint32_t)i;
+    }
+    __syncthreads();
+    // stable within each cell: the rank by previous index
+#pragma unroll
+    for (int u = 0; u < kSortPer; ++u) {
+        const int i = tid + u * kSortThreads;
+        if (i >= n) continue;
+        const uint32_t st = cnt[key[u]], en = cnt[key[u] + 1];
+        uint32_t r = st;
+        for (uint32_t q = st; q < en; ++q) r += perm[q] < (uint32_t)i ? 1u : 0u;
+        const int dst = S.p_off + (int)r;
+        a.spos[dst] = x[u];
+        a.svel[dst] = v[u];
+        if (S.flags & kFlagRecord) a.snbid[dst] = a.nbid[S.p_off + i];
+    }
+}
+
 // Where entry q of the neighbour list of lane l of a tile of T particles is,
 // from the tile's start: groups of four entries, the lanes' groups side by
 // side.
@@ -2595,6 +2665,14 @@ void launch(bool early, void (*k)(P...), int grid, int block, size_t smem, cudaS
 
 }  // namespace
 
+void launch_sort_small(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
+    launch(s.early, k_sort_small, s.grid_p, kSortThreads, s.sort_smem, st, a);
+}
+size_t sort_small_smem(int64_t max_n, int64_t max_keys) {
+    const int64_t per = ((max_keys + kSortThreads - 1) / kSortThreads) | 1;
+    const int64_t bytes = (kSmallSort + per * kSortThreads) * 4;
+    return max_n <= kSmallSort && bytes <= kSmallSortBytes ? (size_t)bytes : 0;
+}
 void launch_keys(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     launch(s.early, k_keys, (s.grid_p + kKeyTiles - 1) / kKeyTiles, s.tile, 0, st, a);
 }
@@ -2681,6 +2759,7 @@ void launch_gather_by_id(const float4* pos, const float4* vel, const float4* dyn
 
 void configure_kernels() {
     const int bytes = kListCap * kMaxTile * (int)sizeof(uint32_t);
+    cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSortBytes);
     cudaFuncSetAttribute(k_density<false, true, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     cudaFuncSetAttribute(k_density<false, true, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     cudaFuncSetAttribute(k_force<false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);

@@ -66,6 +66,11 @@ struct DevArrays {
 // Slots per particle of the in-range neighbour lists.
 constexpr int kNbCap = 192;
 
+// The one-block sort of small scenes: most particles, and most shared memory
+// (counts for 49,000 keys beside the order).
+constexpr int kSmallSort = 4096;
+constexpr int kSmallSortBytes = 215040;
+
 struct LaunchShape {
     int tile;        // threads per particle tile
     int grid_p;      // persistent grid of particle kernels
@@ -73,6 +78,7 @@ struct LaunchShape {
     int grid_t;      // persistent grid of the terrain kernel
     int variant;     // sph_system_config.variant bits (bit 3 only with lists allocated)
     bool pack;       // the density pass writes packed records, the force pass gathers them
+    size_t sort_smem;  // shared memory of the one-block sort; 0: a scene is too large for it
     bool early;      // few particles: each kernel's launch overlaps the kernel before it
     bool density_group, force_group, ordered_group;  // few particles: a group of lanes per particle (group_rules)
     bool record;     // some scene keeps its force records (SPH_FLAG_RECORD)
@@ -83,6 +89,10 @@ struct LaunchShape {
 // Once per process and device: opt the list-traversal kernels into >48 KB of
 // dynamic shared memory.
 void configure_kernels();
+// Shared memory of the one-block sort for scenes of at most max_n particles and
+// max_keys keys; 0: too large for it.
+size_t sort_small_smem(int64_t max_n, int64_t max_keys);
+void launch_sort_small(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_keys(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_scan(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_scatter(const DevArrays& a, const LaunchShape& s, cudaStream_t st);

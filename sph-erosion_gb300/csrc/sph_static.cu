@@ -75,6 +75,8 @@ unsigned char* scratch_for_current_device() {
     if (!g_addr[dev]) {
         void* p = nullptr;
         check_cuda(cudaGetSymbolAddress(&p, g_scratch), "cudaGetSymbolAddress(g_scratch)");
+        configure_kernels();  // shared-memory opt-ins of the kernels, per device
+        check_cuda(cudaGetLastError(), "configure_kernels");
         g_addr[dev] = static_cast<unsigned char*>(p);
     }
     return g_addr[dev];
@@ -192,6 +194,7 @@ extern "C" SPH_API int sph_density_static(const sph_params* p, int n, const floa
         s.variant = 0;
         s.pack = false;
         s.early = true;
+        s.sort_smem = sort_small_smem(n, sc.k_cap);
         s.ordered_group = false;
         s.density_group = true;  // at most 32,768 particles (group_rules)
         s.force_group = true;    // no list is written
@@ -201,10 +204,14 @@ extern "C" SPH_API int sph_density_static(const sph_params* p, int n, const floa
 
         const int nb = (n + 255) / 256;
         k_pack<<<nb, 256, 0, st>>>(pos3_dev, n, a.pos, a.vel);
-        launch_keys(a, s, st);
-        launch_scan(a, s, st);
-        launch_scatter(a, s, st);
-        launch_reorder(a, s, st);
+        if (s.sort_smem) {
+            launch_sort_small(a, s, st);
+        } else {
+            launch_keys(a, s, st);
+            launch_scan(a, s, st);
+            launch_scatter(a, s, st);
+            launch_reorder(a, s, st);
+        }
         launch_density(a, s, st);
         k_unpack<<<nb, 256, 0, st>>>(a.spos, a.dyn, n, density_dev, pressure_dev);
         check_cuda(cudaGetLastError(), "launch");

@@ -102,3 +102,28 @@ def test_ordered_lists_bit_exact(cell_mult):
     for fill in (0, 40000):
         with pytest.raises(S.SphError):
             ordered([129, 3], cell_mult, fill)
+
+
+@pytest.mark.parametrize("cell_mult", [1.0, 0.25])
+@pytest.mark.parametrize("n", [1, 33, 1023, 1024, 1025, 4095, 4096, 4097])
+def test_one_block_sort(n, cell_mult):
+    """The one-block sort of small scenes gives the keys, the stable order and
+    the state after two steps of the sort over the whole system (taken when
+    another scene is larger); grids of 1,000 to 60,000 keys."""
+    rng = np.random.default_rng(n)
+    pos = rng.uniform(-0.19, 0.19, (n, 3)).astype(np.float32)
+    pos[: n // 7] = pos[0]  # a full cell
+    vel = rng.normal(0.0, 0.3, pos.shape).astype(np.float32)
+    out = []
+    for fill in (0, 5000):
+        with S.System(particle_capacity=n + fill) as sysm:
+            prm = dict(REF, cell_mult=cell_mult)
+            sc = sysm.scene(S.default_params(**prm, flags=S.SPH_FLAG_RECORD), capacity=n)
+            sc.set_particles(pos, vel)
+            if fill:
+                sysm.scene(S.default_params(**prm)).set_particles(rng.uniform(-0.19, 0.19, (fill, 3)))
+            sort = sc.debug_sort()
+            sysm.step(2)
+            out.append((*sort, *sc.get_records(), sc.debug_sort()[1]))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b, equal_nan=a.dtype.kind == "f")
