@@ -1192,6 +1192,7 @@ DevArrays System::arrays() const {
     a.status = status_.p;
     a.ctr = status_.p + 1;
     a.tile = cfg_.tile;
+    a.early = false;
     return a;
 }
 

@@ -35,7 +35,8 @@ constexpr unsigned kFull = 0xffffffffu;
 // of the previous kernel's have started, and wait here until it has completed
 // and its writes are visible.  Every thread of every kernel of the step calls
 // this first: a kernel that has completed implies that all before it have.
-__device__ __forceinline__ void step_enter() {
+__device__ __forceinline__ void step_enter(bool early) {
+    if (!early) return;  // not launched that way: the instructions are not free (terrain kernel 31 vs 21 us)
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
@@ -586,7 +587,7 @@ __device__ __forceinline__ Run run_of(uint32_t v, unsigned mask, int lane) {
 constexpr int kKeyTiles = 4;
 
 __global__ void __launch_bounds__(kMaxTile) k_keys(DevArrays a) {
-    step_enter();
+    step_enter(a.early);
     const int nwork = *a.n_ptiles;
     const int lane = threadIdx.x & 31;
     for (int w0 = blockIdx.x * kKeyTiles; w0 < nwork; w0 += gridDim.x * kKeyTiles) {
@@ -676,7 +677,7 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* sh) {
 // chunk totals of its scene, so no block waits on another.  Counts are
 // cleared for the next step.
 __global__ void __launch_bounds__(kScanThreads) k_scan(DevArrays a) {
-    step_enter();
+    step_enter(a.early);
     __shared__ uint32_t sh[kScanThreads / 32];
     const int nwork = *a.n_ctiles;
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
@@ -719,7 +720,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(DevArrays a) {
 // scatter: place each particle's index at its cell's offset + slot, and clear
 // the chunk totals (the scan that read them has finished).
 __global__ void __launch_bounds__(kMaxTile) k_scatter(DevArrays a) {
-    step_enter();
+    step_enter(a.early);
     const int nwork = *a.n_ptiles;
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
         const Work wk = a.ptiles[w];
@@ -744,7 +745,7 @@ __global__ void __launch_bounds__(kMaxTile) k_scatter(DevArrays a) {
 // so results never depend on atomic arrival order) and gather the state into
 // the sorted arrays.
 __global__ void __launch_bounds__(kMaxTile) k_reorder(DevArrays a) {
-    step_enter();
+    step_enter(a.early);
     const int nwork = *a.n_ptiles;
     if (a.ctr && blockIdx.x == 0 && threadIdx.x < 2) a.ctr[threadIdx.x] = 0u;  // for this step's neighbour kernels
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
@@ -783,7 +784,7 @@ constexpr int kSortThreads = 1024;
 constexpr int kSortPer = kSmallSort / kSortThreads;  // particles a thread takes
 
 __global__ void __launch_bounds__(kSortThreads) k_sort_small(const __grid_constant__ DevArrays a) {
-    step_enter();
+    step_enter(a.early);
     extern __shared__ uint32_t sm[];
     __shared__ uint32_t s_warp[kSortThreads / 32];
     const int tid = threadIdx.x;
@@ -877,7 +878,7 @@ __device__ __forceinline__ int first_slice(unsigned* ctr) {
 // neighbour density, so the autotuner picks it.
 template <bool ORDERED, bool LISTED, int MINB>
 __global__ void __launch_bounds__(kMaxTile, MINB) k_density(DevArrays a) {
-    step_enter();
+    step_enter(a.early);
     extern __shared__ uint32_t list[];
     const int nwork = *a.n_ptiles;
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
@@ -992,8 +993,10 @@ __device__ __forceinline__ void for_rows_ahead(const DevArrays& a, const SceneDe
     }
 }
 
-// Entries of a lane's buffer (ListOut).
-constexpr int kBuf = 24;
+// Entries of a lane's buffer (ListOut), which is emptied, and read to its end, in
+// groups of four.
+constexpr int kBuf = 28;
+static_assert(kBuf % 4 == 0 && kBuf >= 8, "whole groups, and room for four beside one");
 
 // One lane's neighbour list while it is written.  The lanes of a warp are at
 // different entries, so an index stored by itself is four bytes to a sector of
@@ -1001,9 +1004,9 @@ constexpr int kBuf = 24;
 // half of the L1-to-L2 path's time, and L2 wrote some of them out half filled
 // (DRAM 406 MB written for 280).  Here the indices go to the lane's column of
 // a buffer in shared memory and from there to the list in groups of four, all
-// lanes together: 3,291 -> 2,719 us for the 8.4M rain in fast arithmetic.  24
-// entries a lane: 16 empty it too often (2,785), 40 leave the candidates too
-// little L1 (2,995).
+// lanes together: 3,291 -> 2,672 us for the 8.4M rain in fast arithmetic.  28
+// entries a lane: 16 empty it too often (2,824), 24 take 2,703; the buffer is
+// sized by the tile, since what it takes is lost to the candidates' L1.
 struct ListOut {
     uint32_t* nl;      // the lane's group 0
     uint32_t stride;   // words from one of its groups to the next
@@ -1135,11 +1138,11 @@ __device__ __forceinline__ float density_sum_exact(const DevArrays& a, const Sce
 // but leaves 40% of the lanes waiting for the longest row.  80 registers: at 64
 // the compiler spills (fast 437 instead of 328 us), 16 warps an SM are too few
 // (392).  1,048,576 particles, before and after: fast, cells of h/2, 380 ->
-// 318 us; exact, cells of h, 488 -> 444 us.
+// 315 us; exact, cells of h, 488 -> 439 us.
 template <bool FM>
 __global__ void __launch_bounds__(kMaxTile, 3) k_density_list(const __grid_constant__ DevArrays a, bool pack) {
-    step_enter();
-    __shared__ uint32_t buf[kMaxTile / 32][kBuf][32];
+    step_enter(a.early);
+    extern __shared__ uint32_t buf[];  // kBuf x 32 words a warp
     const int nwork = *a.n_ptiles;
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
         const Work wk = a.ptiles[w];
@@ -1150,7 +1153,7 @@ __global__ void __launch_bounds__(kMaxTile, 3) k_density_list(const __grid_const
         const bool valid = p < S.p_off + S.n;
         const float4 xi = a.spos[valid ? p : S.p_off];
         const float4* sp = a.spos + S.p_off;
-        uint32_t* col = &buf[threadIdx.x >> 5][0][threadIdx.x & 31];
+        uint32_t* col = buf + (threadIdx.x >> 5) * (kBuf * 32) + (threadIdx.x & 31);
         ListOut out = {a.nlist + (size_t)wk.start * kNbCap + 4 * threadIdx.x, 4 * blockDim.x, col, col, 0};
         float rho = 0.0f;
         const f2 nzero = neg_zero();
@@ -1282,7 +1285,7 @@ __device__ __forceinline__ void integrate_and_store(const DevArrays& a, const Sc
 // systems whose HBM budget has no room for the packed records (k_force_rec).
 template <bool ORDERED, int MINB, bool NL = false, bool DYN = false, bool FM = false>
 __global__ void __launch_bounds__(kMaxTile, MINB) k_force(DevArrays a) {
-    step_enter();
+    step_enter(a.early);
     extern __shared__ uint32_t list[];
     const int nwork = *a.n_ptiles;
     const int spt = DYN ? a.tile / 32 : 1;  // slices per tile
@@ -1518,7 +1521,7 @@ __device__ __noinline__ void force_cells(const DevArrays& a, const SceneDev& S, 
 // faster with 32 warps and no records in flight (364 vs 375 us).
 template <bool FM, bool REC>
 __global__ void __launch_bounds__(kMaxTile, FM ? 3 : 4) k_force_rec(const __grid_constant__ DevArrays a) {
-    step_enter();
+    step_enter(a.early);
     const int nwork = *a.n_ptiles;
     const int spt = a.tile / 32;
     for (int sl = first_slice<true>(a.ctr + 1); sl < nwork * spt; sl = next_slice<true>(a.ctr + 1, sl)) {
@@ -1762,7 +1765,7 @@ __device__ __forceinline__ void density_coop_particle(const DevArrays& a, const 
 
 template <int G, bool PACK>
 __global__ void __launch_bounds__(256) k_density_coop(DevArrays a) {
-    step_enter();
+    step_enter(a.early);
     __shared__ int s_off[256];
     const Group<G> g;
     int* soff = s_off + (threadIdx.x & ~(G - 1));
@@ -1793,7 +1796,7 @@ __global__ void __launch_bounds__(256) k_density_coop(DevArrays a) {
 // overflowed has the group split its cell rows instead (row r to lane r mod G).
 template <int G, bool PACK, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_force_coop(DevArrays a) {
-    step_enter();
+    step_enter(a.early);
     const Group<G> g;
     const int group = threadIdx.x / G, ngroups = blockDim.x / G;
     const int nwork = *a.n_ptiles;
@@ -2010,7 +2013,7 @@ __device__ __forceinline__ void density_group_particle(const DevArrays& a, const
 template <bool FM>
 __global__ void __launch_bounds__(256, 5) k_density_group(const __grid_constant__ DevArrays a, bool lane_lists,
                                                           bool pack) {
-    step_enter();
+    step_enter(a.early);
     constexpr int G = 32, N = 256 / G;
     __shared__ int s_off[256];
     __shared__ float s_term[N][kTerms + 1];
@@ -2109,7 +2112,7 @@ __device__ __forceinline__ void pair_values(const SceneDev& S, float rx, float r
 
 template <bool FM, bool REC>
 __global__ void __launch_bounds__(256, 4) k_force_group(const __grid_constant__ DevArrays a) {
-    step_enter();
+    step_enter(a.early);
     constexpr int G = 16, N = 256 / G, V = kPairValues<FM>, W = G + 1;
     __shared__ float s_val[N][V][W];
     __shared__ float s_sum[N][13];  // the ten sums, NeighbId, whether there is a neighbour; the particle
@@ -2245,7 +2248,7 @@ __device__ __forceinline__ int ordered_particle(const DevArrays& a, int wid, Wor
 }
 
 __global__ void __launch_bounds__(256) k_density_ordered(const __grid_constant__ DevArrays a) {
-    step_enter();
+    step_enter(a.early);
     __shared__ int s_off[8][32];
     __shared__ OrderedList s_list[8];
     const Group<32> g;
@@ -2275,7 +2278,7 @@ __global__ void __launch_bounds__(256) k_density_ordered(const __grid_constant__
 }
 
 __global__ void __launch_bounds__(256) k_force_ordered(const __grid_constant__ DevArrays a) {
-    step_enter();
+    step_enter(a.early);
     constexpr int V = kPairValues<false>;
     __shared__ int s_off[8][32];
     __shared__ OrderedList s_list[8];
@@ -2396,7 +2399,7 @@ __device__ __forceinline__ void tma_gather4(void* dst, const CUtensorMap* map, i
 
 template <int MINB>
 __global__ void __launch_bounds__(kMaxTile + 32, MINB) k_force_tma(DevArrays a, const __grid_constant__ CUtensorMap fmap) {
-    step_enter();
+    step_enter(a.early);
     extern __shared__ unsigned char smem_raw[];
     __shared__ int s_m;
     const int T = (int)blockDim.x - 32;  // consumers: 128 or 256
@@ -2516,15 +2519,18 @@ size_t force_tma_smem(int tile) {
 // terrain: height snapshot = base + delta * unit, read by the next step.
 // Four vertices per thread: a tile of T vertices takes T / 4 threads, each
 // with 16-byte loads and stores (a scene's vertices start on a 512-vertex
-// boundary, so every thread's first vertex is 4-aligned).
-__global__ void __launch_bounds__(kMaxTile / 4) k_terrain(DevArrays a) {
-    step_enter();
-    const int nwork = *a.n_ttiles;
-    for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
+// boundary, so every thread's first vertex is 4-aligned).  A block takes 1024 /
+// T tiles: with one tile, a warp or two, the blocks' own overhead was a third
+// of the time (16.8 million vertices, tile 128: 72 -> 45 us, 7.4 TB/s).
+__global__ void __launch_bounds__(256) k_terrain(DevArrays a) {
+    step_enter(a.early);
+    const int nwork = *a.n_ttiles, T4 = a.tile / 4, per = 256 / T4;
+    const int sub = threadIdx.x / T4, lane = threadIdx.x % T4;
+    for (int w = blockIdx.x * per + sub; w < nwork; w += gridDim.x * per) {
         const Work wk = a.ttiles[w];
         if (a.steps_left[wk.scene] == 0) continue;
         const SceneDev& S = a.scenes[wk.scene];
-        const int t = wk.start + 4 * (int)threadIdx.x;
+        const int t = wk.start + 4 * lane;
         const int end = S.t_off + S.tw * S.td;
         const float u = S.height_unit;
         if (t + 3 < end) {
@@ -2540,8 +2546,8 @@ __global__ void __launch_bounds__(kMaxTile / 4) k_terrain(DevArrays a) {
     }
 }
 
-__global__ void k_tick(int* steps_left, int nscenes) {
-    step_enter();
+__global__ void k_tick(int* steps_left, int nscenes, bool early) {
+    step_enter(early);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < nscenes && steps_left[s] > 0) steps_left[s] -= 1;
 }
@@ -2648,8 +2654,20 @@ __global__ void __launch_bounds__(256) k_diag(DevArrays a, double* partial, long
 // us, with and without: 100,000 particles 127 vs 113, 1,048,576 862 vs 818,
 // 8.4M 5,367 vs 4,949): the list passes keep the L1 split of the kernel they
 // overlapped.
+template <class T>
+T with_early(T v, bool) {
+    return v;
+}
+DevArrays with_early(DevArrays a, bool early) {
+    a.early = early;  // tells the kernel to wait
+    return a;
+}
 template <class... P, class... A>
 void launch(bool early, void (*k)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args) {
+    if (!early) {
+        k<<<grid, block, smem, st>>>(P(with_early(args, early))...);
+        return;
+    }
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3((unsigned)grid);
     c.blockDim = dim3((unsigned)block);
@@ -2659,8 +2677,8 @@ void launch(bool early, void (*k)(P...), int grid, int block, size_t smem, cudaS
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     c.attrs = &at;
-    c.numAttrs = early ? 1 : 0;
-    cudaLaunchKernelEx(&c, k, P(args)...);
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, k, P(with_early(args, early))...);
 }
 
 }  // namespace
@@ -2882,9 +2900,9 @@ void launch_density(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
         launch_density_group(a, s, (s.variant & 131072) != 0, st);
     } else if (s.variant & 8) {
         if (s.variant & 131072)
-            launch(s.early, k_density_list<true>, s.grid_p, s.tile, 0, st, a, s.pack);
+            launch(s.early, k_density_list<true>, s.grid_p, s.tile, (size_t)s.tile * kBuf * 4, st, a, s.pack);
         else
-            launch(s.early, k_density_list<false>, s.grid_p, s.tile, 0, st, a, s.pack);
+            launch(s.early, k_density_list<false>, s.grid_p, s.tile, (size_t)s.tile * kBuf * 4, st, a, s.pack);
     } else if (s.variant & 1) {
         if (relaxed)
             launch(s.early, k_density<false, true, 4>, s.grid_p, s.tile, list_bytes(s), st, a);
@@ -2949,10 +2967,10 @@ void launch_force_ordered(const DevArrays& a, const LaunchShape& s, cudaStream_t
         launch(s.early, k_force<true, 1>, s.grid_p, s.tile, 0, st, a);
 }
 void launch_terrain(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    launch(s.early, k_terrain, s.grid_t, s.tile / 4, 0, st, a);
+    launch(s.early, k_terrain, (s.grid_t * (s.tile / 4) + 255) / 256, 256, 0, st, a);
 }
 void launch_tick(const DevArrays& a, const LaunchShape& s, int nscenes, cudaStream_t st) {
-    launch(s.early, k_tick, (nscenes + 127) / 128, 128, 0, st, a.steps_left, nscenes);
+    launch(s.early, k_tick, (nscenes + 127) / 128, 128, 0, st, a.steps_left, nscenes, s.early);
 }
 void launch_neighbour_counts(const DevArrays& a, const LaunchShape& s, int32_t* out_by_id, cudaStream_t st) {
     k_neighbour_counts<<<s.grid_p, s.tile, 0, st>>>(a, out_by_id);

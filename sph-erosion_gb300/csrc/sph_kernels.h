@@ -61,6 +61,7 @@ struct DevArrays {
     // null where no kernel is scheduled that way
     unsigned* ctr;
     int tile;      // lanes per work tile (the list stride)
+    bool early;    // set by the launchers: the kernel overlaps the one before it and waits for it
 };
 
 // Slots per particle of the in-range neighbour lists.
