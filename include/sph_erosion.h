@@ -113,15 +113,17 @@ typedef struct sph_system_config {
     int graph_steps;          /* steps per captured CUDA graph (0 = no graphs) */
     int variant;              /* kernel variant bits, picked by the autotuner:
                                  1 = density pass over compacted neighbour lists,
-                                 4 = relaxed register budget (fewer resident blocks),
+                                 4 = relaxed register budget (fewer resident blocks;
+                                     the list passes of 8 have their own and ignore it),
                                  8 = the density pass writes each particle's in-range
                                      neighbours (192 slots, 772 B per particle) and the
                                      force pass reads them instead of re-testing the
                                      cells; ignored when the HBM budget has no room,
                                 16 = with 8: the force pass's list walk loads ahead (every
                                      list walk does now; fast arithmetic still asks for it),
-                                32 = with 8: relaxed register budget of the density pass only,
-                                64 = with 8: the density pass loads candidates in pairs,
+                                32 = with 8: was the density pass's relaxed register budget,
+                                64 = with 8: was its paired candidate loads (one list-writing
+                                     density pass serves every per-lane form now),
                                128 = with 8: the force pass gathers one packed 32-byte
                                      record per neighbour (32 more bytes per particle,
                                      part of the variant's memory; without the bit they
@@ -133,7 +135,8 @@ typedef struct sph_system_config {
                                      with 256, bit 4 relaxes the force pass's registers,
                              32768 = with 8 + 16: the force pass's warps take their work
                                      in 32-particle slices from a counter (they always do
-                                     now; 65536: the density pass's); same bits,
+                                     now; 65536, the density pass's, has no effect with 8);
+                                     same bits,
                             131072 = with 8 + 16: fast arithmetic in both neighbour passes
                                      (grouped products, fused multiply-adds, r^2 for
                                      |r|^2, hardware 1/sqrt); exact in-range test, so the
@@ -165,7 +168,9 @@ SPH_API int sph_system_sync(sph_system* s);  /* waits for steps and asynchronous
 /* Device time of nsteps steps measured with CUDA events on the system stream. */
 SPH_API int sph_system_time_steps(sph_system* s, int nsteps, float* ms);
 /* Device time per stage of one step, averaged over nsteps (stages: keys, scan,
- * scatter, reorder, density, force, terrain, tick); ms must hold 8 floats. */
+ * scatter, reorder, density, force, terrain, tick); ms must hold 8 floats.
+ * Small scenes (4,096 particles, about 49,000 grid keys) are sorted by one
+ * kernel, timed under keys. */
 SPH_API int sph_system_profile_stages(sph_system* s, int nsteps, float* ms);
 /* Bytes of device memory the system holds. */
 SPH_API int sph_system_memory(sph_system* s, int64_t* bytes);

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 import sph_gb300 as S
-from helpers import REF
+from helpers import REF, height_unit
 
 pytestmark = pytest.mark.gpu
 
@@ -127,3 +127,25 @@ def test_one_block_sort(n, cell_mult):
             out.append((*sort, *sc.get_records(), sc.debug_sort()[1]))
     for a, b in zip(*out):
         assert np.array_equal(a, b, equal_nan=a.dtype.kind == "f")
+
+
+@pytest.mark.parametrize("tile", [128, 256])
+@pytest.mark.parametrize("shape", [(2, 2), (16, 8), (43, 3), (32, 28), (32, 32), (35, 33), (64, 65)])
+def test_terrain_snapshot_of_every_tile(shape, tile):
+    """The height snapshot is base + delta * unit at every vertex when the
+    vertices are one tile or less, one more than a tile, and fill, underfill
+    and overrun a block of several tiles."""
+    rng = np.random.default_rng(5)
+    base = rng.uniform(0.0, 0.1, shape[::-1]).astype(np.float32)
+    pos = np.stack(np.meshgrid(*[np.linspace(-0.18, 0.18, 40)] * 2), -1).reshape(-1, 2)
+    pos = np.insert(pos, 1, -0.15, axis=1).astype(np.float32)
+    prm = dict(REF, dt=1e-3, erosion=1, k_capacity=0.05, erosion_layer=0.2)
+    with S.System(tile=tile) as sysm:
+        sc = sysm.scene(S.default_params(**prm), capacity=len(pos), terrain=shape)
+        sc.set_terrain(base)
+        sc.set_particles(pos, rng.normal(0.0, 1.0, pos.shape).astype(np.float32))
+        sysm.step(3)
+        h, delta = sc.get_terrain()
+        assert sc.diag()["total_units"] == 0
+    assert np.count_nonzero(delta) > delta.size // 8
+    assert np.array_equal(h, base + delta.astype(np.float32) * height_unit(prm, shape))
