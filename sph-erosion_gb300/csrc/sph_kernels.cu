@@ -559,8 +559,7 @@ __device__ __forceinline__ float len3(float x, float y, float z) { return fsq(di
 // prefix, `mask`): the first lane of each run adds the run's length to
 // counter[v] and every lane gets old value + its position in the run.  The
 // state arrives in the previous step's sorted order, so particles of one cell
-// are mostly adjacent and one atomic serves each cell.  Split in three phases
-// so that several independent runs can have their atomics in flight at once.
+// are mostly adjacent and one atomic serves each cell.
 struct Run {
     bool start;
     int leader;
@@ -581,64 +580,53 @@ __device__ __forceinline__ Run run_of(uint32_t v, unsigned mask, int lane) {
 }
 
 // keys: cell key of each particle, its slot within the cell (run-aggregated
-// atomics) and the per-chunk totals that the scan needs.  Each block takes
-// kKeyTiles consecutive work items, with their loads, then their atomics,
-// then their shuffles issued together.
-constexpr int kKeyTiles = 4;
-
+// atomics) and the per-chunk totals that the scan needs.  The particles of a
+// block are nearly all of one chunk, so the block adds that chunk's total once
+// and only strays go to memory one by one: a system has a few hundred chunks, on
+// a few dozen sectors, and an add per warp queued there (1,048,576 particles:
+// 32,768 adds; keys of cells of h 33 -> 16 us, of h/2 29 -> 17; 8.4M rain 140 ->
+// 81).  One tile a block: with the queue gone, four with their loads together
+// are slower (20, 21, 90 us).
 __global__ void __launch_bounds__(kMaxTile) k_keys(DevArrays a) {
     step_enter(a.early);
+    __shared__ uint32_t s_chunk, s_sum;
     const int nwork = *a.n_ptiles;
     const int lane = threadIdx.x & 31;
-    for (int w0 = blockIdx.x * kKeyTiles; w0 < nwork; w0 += gridDim.x * kKeyTiles) {
-        bool valid[kKeyTiles];
-        int idx[kKeyTiles];
-        uint32_t k[kKeyTiles], gk[kKeyTiles], ck[kKeyTiles];
-        float4 x[kKeyTiles];
-#pragma unroll
-        for (int u = 0; u < kKeyTiles; ++u) {
-            valid[u] = false;
-            idx[u] = 0;
-            const int w = w0 + u;
-            if (w < nwork) {
-                const Work wk = a.ptiles[w];
-                if (a.steps_left[wk.scene] != 0) {
-                    const SceneDev& S = a.scenes[wk.scene];
-                    idx[u] = wk.start + threadIdx.x;
-                    valid[u] = idx[u] < S.p_off + S.n;
-                    if (valid[u]) x[u] = a.pos[idx[u]];
-                }
+    for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
+        const Work wk = a.ptiles[w];
+        if (a.steps_left[wk.scene] == 0) continue;
+        const SceneDev& S = a.scenes[wk.scene];
+        const int i = wk.start + threadIdx.x;
+        const bool valid = i < S.p_off + S.n;
+        const unsigned mask = __ballot_sync(kFull, valid);
+        uint32_t k = 0, ck = 0;
+        if (valid) {
+            const float4 x = a.pos[i];
+            const Cell c = cell_of(S, x.x, x.y, x.z);
+            k = row_key(a.tab, S, c.cy, c.cz) + (uint32_t)c.cx;
+            ck = k >> kChunkBits;
+        }
+        if (threadIdx.x == 0) {  // a tile's first particle is valid
+            s_chunk = ck;
+            s_sum = 0u;
+        }
+        __syncthreads();
+        if (valid) {
+            const Run r = run_of(k, mask, lane);
+            uint32_t base = 0;
+            if (r.start) base = atomicAdd(a.counts + S.k_off + k, r.len);
+            const Run rc = run_of(ck, mask, lane);
+            if (rc.start) {
+                if (ck == s_chunk)
+                    atomicAdd(&s_sum, rc.len);
+                else
+                    atomicAdd(a.chunk_sum + S.c_off + ck, rc.len);
             }
+            a.key[i] = k;
+            a.slot[i] = __shfl_sync(mask, base, r.leader) + (uint32_t)(lane - r.leader);
         }
-#pragma unroll
-        for (int u = 0; u < kKeyTiles; ++u) {
-            if (!valid[u]) continue;
-            const SceneDev& S = a.scenes[a.ptiles[w0 + u].scene];
-            const Cell c = cell_of(S, x[u].x, x[u].y, x[u].z);
-            k[u] = row_key(a.tab, S, c.cy, c.cz) + (uint32_t)c.cx;
-            gk[u] = (uint32_t)S.k_off + k[u];
-            ck[u] = (uint32_t)S.c_off + (k[u] >> kChunkBits);
-        }
-        Run rk[kKeyTiles];
-        uint32_t base[kKeyTiles];
-#pragma unroll
-        for (int u = 0; u < kKeyTiles; ++u) {
-            const unsigned mask = __ballot_sync(kFull, valid[u]);
-            base[u] = 0;
-            if (!valid[u]) continue;
-            rk[u] = run_of(gk[u], mask, lane);
-            const Run rc = run_of(ck[u], mask, lane);
-            if (rk[u].start) base[u] = atomicAdd(a.counts + gk[u], rk[u].len);
-            if (rc.start) atomicAdd(a.chunk_sum + ck[u], rc.len);
-        }
-#pragma unroll
-        for (int u = 0; u < kKeyTiles; ++u) {
-            const unsigned mask = __ballot_sync(kFull, valid[u]);
-            if (!valid[u]) continue;
-            const uint32_t b = __shfl_sync(mask, base[u], rk[u].leader);
-            a.key[idx[u]] = k[u];
-            a.slot[idx[u]] = b + (uint32_t)(lane - rk[u].leader);
-        }
+        __syncthreads();
+        if (threadIdx.x == 0) atomicAdd(a.chunk_sum + S.c_off + ck, s_sum);
     }
 }
 
@@ -1136,7 +1124,7 @@ __device__ __forceinline__ float density_sum_exact(const DevArrays& a, const Sce
 // a pair to evaluate.  No unit bounds it (instructions 65%, L1 data path 60%):
 // the rows are walked in step, which keeps a warp's loads in few cache lines
 // but leaves 40% of the lanes waiting for the longest row.  80 registers: at 64
-// the compiler spills (fast 437 instead of 328 us), 16 warps an SM are too few
+// the compiler spills (437 where these take 327 us), 16 warps an SM are too few
 // (392).  1,048,576 particles, before and after: fast, cells of h/2, 380 ->
 // 315 us; exact, cells of h, 488 -> 439 us.
 template <bool FM>
@@ -1514,11 +1502,12 @@ __device__ __noinline__ void force_cells(const DevArrays& a, const SceneDev& S, 
 // cycles, 71% of the fast form's time; taking neighbours in pairs cut the
 // other part, the instructions (227 to 137 million a launch at 1,048,576
 // particles, 56 in range), and with them the time from 351 to 270 us (exact
-// arithmetic 447 to 364, with the packed records in place of three arrays).
-// The fast form loads the records of the next pair before it sums the current
-// one, at 80 registers and 24 warps an SM (without: 281 us at 64 registers,
-// 309 at 80); the exact form, with more arithmetic between its loads, is
-// faster with 32 warps and no records in flight (364 vs 375 us).
+// arithmetic 447 to 364, with the packed records in place of three arrays);
+// list entries read two to a load brought 240 and 353.  The fast form loads
+// the records of the next pair before it sums the current one, at 80 registers
+// and 24 warps an SM (without, entries still read one by one: 281 us at 64
+// registers, 309 at 80); the exact form, with more arithmetic between its
+// loads, is faster with 32 warps and no records in flight (364 vs 375 us).
 template <bool FM, bool REC>
 __global__ void __launch_bounds__(kMaxTile, FM ? 3 : 4) k_force_rec(const __grid_constant__ DevArrays a) {
     step_enter(a.early);
@@ -2692,7 +2681,7 @@ size_t sort_small_smem(int64_t max_n, int64_t max_keys) {
     return max_n <= kSmallSort && bytes <= kSmallSortBytes ? (size_t)bytes : 0;
 }
 void launch_keys(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    launch(s.early, k_keys, (s.grid_p + kKeyTiles - 1) / kKeyTiles, s.tile, 0, st, a);
+    launch(s.early, k_keys, s.grid_p, s.tile, 0, st, a);
 }
 void launch_scan(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     launch(s.early, k_scan, s.grid_c, kScanThreads, 0, st, a);
