@@ -2864,7 +2864,8 @@ static void launch_force_group(const DevArrays& a, const LaunchShape& s, bool fa
 // 38.3; fast, density 8,000 19.7 vs 24.1, 12,000 24.5 vs 25.7, 16,000 29.0 vs
 // 27.1; fast, force (beside the group density pass) 8,000 19.1 vs 19.7, 12,000
 // 26.5 vs 24.5.  A system alone on the chip gains up to there from 2.3x (1,000
-// particles: 74 to 32 us) to 1.6x (20,000: 99 to 62 us) a step.
+// particles: 74 to 32 us) to 1.6x (20,000: 99 to 62 us) a step (all of this
+// with the sort in four kernels).
 // The ordered passes' line: density + force, us, a warp per particle vs one lane,
 // 5,000 particles 34 vs 127, 16,384 68 vs 143, 50,000 167 vs 217, 200,000 607 vs
 // 536.
