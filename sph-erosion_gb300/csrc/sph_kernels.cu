@@ -30,15 +30,20 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 
 // The kernels of a step follow one another on one stream and each needs all of
-// the one before.  In small systems they are launched with programmatic
-// serialization (launch): a kernel's blocks may then come to the SMs once all
-// of the previous kernel's have started, and wait here until it has completed
-// and its writes are visible.  Every thread of every kernel of the step calls
-// this first: a kernel that has completed implies that all before it have.
+// the one before.  In small systems those that launch() starts early may come
+// to the SMs while the kernel before them runs, and wait here until it has
+// completed and its writes are visible.  Every thread of such a kernel calls
+// this first.  Only then does the kernel let its own dependent start: a
+// dependent is resident beside the one kernel it waits for and never beside an
+// earlier one, whose reads could leave old lines in an L1 that its own reads
+// meet.  While it waits, that kernel writes what it will read, so it takes none
+// of the step's arrays through the non-coherent path (__ldg), which requires
+// them to be constant for a kernel's whole life; the row table is, since only
+// copies write it.
 __device__ __forceinline__ void step_enter(bool early) {
     if (!early) return;  // not launched that way: the instructions are not free (terrain kernel 31 vs 21 us)
-    asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
 }
 
 __device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }
@@ -501,8 +506,8 @@ __device__ __forceinline__ TSample terrain_at(const SceneDev& S, const float* hs
     if (j0 > S.td - 2) j0 = S.td - 2;
     const float tx = fs(fx, (float)i0), tz = fs(fz, (float)j0);
     const float* r0 = hs + S.t_off + (size_t)j0 * S.tw + i0;
-    const float h00 = __ldg(r0), h10 = __ldg(r0 + 1);
-    const float h01 = __ldg(r0 + S.tw), h11 = __ldg(r0 + S.tw + 1);
+    const float h00 = r0[0], h10 = r0[1];
+    const float h01 = r0[S.tw], h11 = r0[S.tw + 1];
     const float a0 = fa(h00, fm(tx, fs(h10, h00)));
     const float a1 = fa(h01, fm(tx, fs(h11, h01)));
     const float hgt = fa(a0, fm(tz, fs(a1, a0)));
@@ -866,7 +871,6 @@ __device__ __forceinline__ int first_slice(unsigned* ctr) {
 // neighbour density, so the autotuner picks it.
 template <bool ORDERED, bool LISTED, int MINB>
 __global__ void __launch_bounds__(kMaxTile, MINB) k_density(DevArrays a) {
-    step_enter(a.early);
     extern __shared__ uint32_t list[];
     const int nwork = *a.n_ptiles;
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
@@ -1129,7 +1133,6 @@ __device__ __forceinline__ float density_sum_exact(const DevArrays& a, const Sce
 // 315 us; exact, cells of h, 488 -> 439 us.
 template <bool FM>
 __global__ void __launch_bounds__(kMaxTile, 3) k_density_list(const __grid_constant__ DevArrays a, bool pack) {
-    step_enter(a.early);
     extern __shared__ uint32_t buf[];  // kBuf x 32 words a warp
     const int nwork = *a.n_ptiles;
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
@@ -1273,7 +1276,6 @@ __device__ __forceinline__ void integrate_and_store(const DevArrays& a, const Sc
 // systems whose HBM budget has no room for the packed records (k_force_rec).
 template <bool ORDERED, int MINB, bool NL = false, bool DYN = false, bool FM = false>
 __global__ void __launch_bounds__(kMaxTile, MINB) k_force(DevArrays a) {
-    step_enter(a.early);
     extern __shared__ uint32_t list[];
     const int nwork = *a.n_ptiles;
     const int spt = DYN ? a.tile / 32 : 1;  // slices per tile
@@ -1473,28 +1475,8 @@ __device__ __forceinline__ void force_one(const SceneDev& S, ForceAcc& acc, cons
         force_pair(S, acc, -q.x, -q.y, -q.z, fsq(q.s), 0.0f, 0.0f, 0.0f, q.AA, dv, 0.0f, q.B, -1, self);
 }
 
-// The neighbour sums of a particle whose list overflowed: it walks its cells
-// (same order).  A call, so that this rare path takes no registers from the
-// list walk.
 template <bool FM>
-__device__ __noinline__ void force_cells(const DevArrays& a, const SceneDev& S, int p, ForceAcc& acc) {
-    const int pl = p - S.p_off;
-    const float4 xi = a.spos[p], vi = a.svel[p], di = a.dyn[p];
-    const float4* sv = a.svel + S.p_off;
-    const float4* sd = a.dyn + S.p_off;
-    for_each_candidate(a, S, xi, [&](uint32_t j, float4 xj) {
-        const float rx = fs(xi.x, xj.x), ry = fs(xi.y, xj.y), rz = fs(xi.z, xj.z);
-        const float s = dist2(rx, ry, rz);
-        if (!(s <= S.smax)) return;
-        const float4 vj = __ldg(sv + j), dj = __ldg(sd + j);
-        if (FM)
-            force_pair_fast(S, acc, rx, ry, rz, dist2_fma(rx, ry, rz), vi.x, vi.y, vi.z, di.y, vj, dj.y, dj.z,
-                            __float_as_int(xj.w), (int)j == pl);
-        else
-            force_pair(S, acc, rx, ry, rz, fsq(s), vi.x, vi.y, vi.z, di.y, vj, dj.y, dj.z, __float_as_int(xj.w),
-                       (int)j == pl);
-    });
-}
+__device__ __noinline__ void force_cells(const DevArrays& a, const SceneDev& S, int p, ForceAcc& acc);
 
 // force over the packed records: the list walk of k_force taken two
 // neighbours at a time, in warp slices from the counter.  The L1 data path
@@ -1510,7 +1492,6 @@ __device__ __noinline__ void force_cells(const DevArrays& a, const SceneDev& S, 
 // loads, is faster with 32 warps and no records in flight (364 vs 375 us).
 template <bool FM, bool REC>
 __global__ void __launch_bounds__(kMaxTile, FM ? 3 : 4) k_force_rec(const __grid_constant__ DevArrays a) {
-    step_enter(a.early);
     const int nwork = *a.n_ptiles;
     const int spt = a.tile / 32;
     for (int sl = first_slice<true>(a.ctr + 1); sl < nwork * spt; sl = next_slice<true>(a.ctr + 1, sl)) {
@@ -1630,14 +1611,45 @@ __device__ __forceinline__ void stencil_row(const DevArrays& a, const SceneDev& 
             if (gx2[RX + d] <= r2) hi = d;
         }
         const uint32_t row = row_key(a.tab, S, y, z);
-        st = __ldg(off + row + q.c.cx + lo);
-        en = __ldg(off + row + q.c.cx + hi + 1);
+        st = off[row + q.c.cx + lo];
+        en = off[row + q.c.cx + hi + 1];
     } else {
         int xl, xh;
         if (!row_span(S, q, y, z, &xl, &xh)) return;
         const uint32_t row = row_key(a.tab, S, y, z);
-        st = __ldg(off + row + xl);
-        en = __ldg(off + row + xh + 1);
+        st = off[row + xl];
+        en = off[row + xh + 1];
+    }
+}
+
+// The neighbour sums of a particle whose list overflowed: it walks its cells
+// (same order).  A call, so that this rare path takes no registers from the
+// list walk.
+template <bool FM>
+__device__ __noinline__ void force_cells(const DevArrays& a, const SceneDev& S, int p, ForceAcc& acc) {
+    const int pl = p - S.p_off;
+    const float4 xi = a.spos[p], vi = a.svel[p], di = a.dyn[p];
+    const float4* sp = a.spos + S.p_off;
+    const float4* sv = a.svel + S.p_off;
+    const float4* sd = a.dyn + S.p_off;
+    const Probe q = probe_of(S, xi);
+    const int side = 2 * S.reach + 1;
+    for (int r = 0; r < side * side; ++r) {
+        uint32_t st, en;
+        stencil_row<0>(a, S, q, nullptr, r, st, en);
+        for (uint32_t j = st; j < en; ++j) {
+            const float4 xj = sp[j];
+            const float rx = fs(xi.x, xj.x), ry = fs(xi.y, xj.y), rz = fs(xi.z, xj.z);
+            const float s = dist2(rx, ry, rz);
+            if (!(s <= S.smax)) continue;
+            const float4 vj = sv[j], dj = sd[j];
+            if (FM)
+                force_pair_fast(S, acc, rx, ry, rz, dist2_fma(rx, ry, rz), vi.x, vi.y, vi.z, di.y, vj, dj.y, dj.z,
+                                __float_as_int(xj.w), (int)j == pl);
+            else
+                force_pair(S, acc, rx, ry, rz, fsq(s), vi.x, vi.y, vi.z, di.y, vj, dj.y, dj.z, __float_as_int(xj.w),
+                           (int)j == pl);
+        }
     }
 }
 
@@ -1754,7 +1766,6 @@ __device__ __forceinline__ void density_coop_particle(const DevArrays& a, const 
 
 template <int G, bool PACK>
 __global__ void __launch_bounds__(256) k_density_coop(DevArrays a) {
-    step_enter(a.early);
     __shared__ int s_off[256];
     const Group<G> g;
     int* soff = s_off + (threadIdx.x & ~(G - 1));
@@ -1785,7 +1796,6 @@ __global__ void __launch_bounds__(256) k_density_coop(DevArrays a) {
 // overflowed has the group split its cell rows instead (row r to lane r mod G).
 template <int G, bool PACK, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_force_coop(DevArrays a) {
-    step_enter(a.early);
     const Group<G> g;
     const int group = threadIdx.x / G, ngroups = blockDim.x / G;
     const int nwork = *a.n_ptiles;
@@ -1938,7 +1948,7 @@ __device__ __forceinline__ int group_walk(const DevArrays& a, const SceneDev& S,
             int id = 0;
             if (t < total) {
                 j = (uint32_t)(t + off);
-                const float4 xj = __ldg(sp + j);
+                const float4 xj = sp[j];
                 s = dist2(fs(xi.x, xj.x), fs(xi.y, xj.y), fs(xi.z, xj.z));
                 in = s <= S.smax;
                 id = __float_as_int(xj.w);
@@ -2144,12 +2154,12 @@ __global__ void __launch_bounds__(256, 4) k_force_group(const __grid_constant__ 
         const int i1 = FM ? (c < 3 ? c : c < 6 ? c + 3 : c < 9 ? c - 3 : 12) : c;
         const int i2 = c < 3 ? 9 : c < 6 ? 10 : c < 9 ? 11 : 13;
         float acc = 0.0f;
-        uint32_t j = c < cnt ? __ldg(nl + c) : pl;
+        uint32_t j = c < cnt ? nl[c] : pl;
         for (int b = 0; b < cnt; b += G) {
-            const float4 xj = __ldg(sp + j), vj = __ldg(sv + j), dj = __ldg(sd + j);
+            const float4 xj = sp[j], vj = sv[j], dj = sd[j];
             const bool live = b + c < cnt, self = j == pl;
             if (REC && live && !self) nb = max(nb, __float_as_int(xj.w)), any = 1;
-            if (b + G + c < cnt) j = __ldg(nl + b + G + c);
+            if (b + G + c < cnt) j = nl[b + G + c];
             if (live) {
                 float v[V];
                 pair_values<FM>(S, fs(xi.x, xj.x), fs(xi.y, xj.y), fs(xi.z, xj.z), fs(vj.x, vi.x), fs(vj.y, vi.y),
@@ -2388,7 +2398,6 @@ __device__ __forceinline__ void tma_gather4(void* dst, const CUtensorMap* map, i
 
 template <int MINB>
 __global__ void __launch_bounds__(kMaxTile + 32, MINB) k_force_tma(DevArrays a, const __grid_constant__ CUtensorMap fmap) {
-    step_enter(a.early);
     extern __shared__ unsigned char smem_raw[];
     __shared__ int s_m;
     const int T = (int)blockDim.x - 32;  // consumers: 128 or 256
@@ -2791,14 +2800,14 @@ static void launch_density_coop(const DevArrays& a, const LaunchShape& s, cudaSt
     const bool pack = (s.variant & 128) != 0;
     if (s.variant & 2048) {
         if (pack)
-            launch(s.early, k_density_coop<16, true>, s.grid_p, s.tile, 0, st, a);
+            k_density_coop<16, true><<<s.grid_p, s.tile, 0, st>>>(a);
         else
-            launch(s.early, k_density_coop<16, false>, s.grid_p, s.tile, 0, st, a);
+            k_density_coop<16, false><<<s.grid_p, s.tile, 0, st>>>(a);
     } else {
         if (pack)
-            launch(s.early, k_density_coop<32, true>, s.grid_p, s.tile, 0, st, a);
+            k_density_coop<32, true><<<s.grid_p, s.tile, 0, st>>>(a);
         else
-            launch(s.early, k_density_coop<32, false>, s.grid_p, s.tile, 0, st, a);
+            k_density_coop<32, false><<<s.grid_p, s.tile, 0, st>>>(a);
     }
 }
 
@@ -2808,19 +2817,19 @@ static void launch_force_coop_b(const DevArrays& a, const LaunchShape& s, cudaSt
     const int gsel = (s.variant >> 9) & 3;
     if (gsel == 1) {
         if (pack)
-            launch(s.early, k_force_coop<4, true, MINB>, s.grid_p, s.tile, 0, st, a);
+            k_force_coop<4, true, MINB><<<s.grid_p, s.tile, 0, st>>>(a);
         else
-            launch(s.early, k_force_coop<4, false, MINB>, s.grid_p, s.tile, 0, st, a);
+            k_force_coop<4, false, MINB><<<s.grid_p, s.tile, 0, st>>>(a);
     } else if (gsel == 2) {
         if (pack)
-            launch(s.early, k_force_coop<16, true, MINB>, s.grid_p, s.tile, 0, st, a);
+            k_force_coop<16, true, MINB><<<s.grid_p, s.tile, 0, st>>>(a);
         else
-            launch(s.early, k_force_coop<16, false, MINB>, s.grid_p, s.tile, 0, st, a);
+            k_force_coop<16, false, MINB><<<s.grid_p, s.tile, 0, st>>>(a);
     } else {
         if (pack)
-            launch(s.early, k_force_coop<8, true, MINB>, s.grid_p, s.tile, 0, st, a);
+            k_force_coop<8, true, MINB><<<s.grid_p, s.tile, 0, st>>>(a);
         else
-            launch(s.early, k_force_coop<8, false, MINB>, s.grid_p, s.tile, 0, st, a);
+            k_force_coop<8, false, MINB><<<s.grid_p, s.tile, 0, st>>>(a);
     }
 }
 
@@ -2890,26 +2899,26 @@ void launch_density(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
         launch_density_group(a, s, (s.variant & 131072) != 0, st);
     } else if (s.variant & 8) {
         if (s.variant & 131072)
-            launch(s.early, k_density_list<true>, s.grid_p, s.tile, (size_t)s.tile * kBuf * 4, st, a, s.pack);
+            k_density_list<true><<<s.grid_p, s.tile, (size_t)s.tile * kBuf * 4, st>>>(a, s.pack);
         else
-            launch(s.early, k_density_list<false>, s.grid_p, s.tile, (size_t)s.tile * kBuf * 4, st, a, s.pack);
+            k_density_list<false><<<s.grid_p, s.tile, (size_t)s.tile * kBuf * 4, st>>>(a, s.pack);
     } else if (s.variant & 1) {
         if (relaxed)
-            launch(s.early, k_density<false, true, 4>, s.grid_p, s.tile, list_bytes(s), st, a);
+            k_density<false, true, 4><<<s.grid_p, s.tile, list_bytes(s), st>>>(a);
         else
-            launch(s.early, k_density<false, true, 8>, s.grid_p, s.tile, list_bytes(s), st, a);
+            k_density<false, true, 8><<<s.grid_p, s.tile, list_bytes(s), st>>>(a);
     } else {
         if (relaxed)
-            launch(s.early, k_density<false, false, 4>, s.grid_p, s.tile, 0, st, a);
+            k_density<false, false, 4><<<s.grid_p, s.tile, 0, st>>>(a);
         else
-            launch(s.early, k_density<false, false, 8>, s.grid_p, s.tile, 0, st, a);
+            k_density<false, false, 8><<<s.grid_p, s.tile, 0, st>>>(a);
     }
 }
 void launch_density_ordered(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     if (s.ordered_group)
         launch(s.early, k_density_ordered, s.grid_p * s.tile / 8, 256, 0, st, a);
     else
-        launch(s.early, k_density<true, false, 1>, s.grid_p, s.tile, 0, st, a);
+        k_density<true, false, 1><<<s.grid_p, s.tile, 0, st>>>(a);
 }
 void launch_force(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     if (coop(s)) {
@@ -2926,35 +2935,35 @@ void launch_force(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     // slices from a counter.
     if (!s.force_group && (s.variant & 262144) && (s.variant & (131072 | 128 | 24)) == (131072 | 128 | 24) && s.fmap) {
         // bit 18: the TMA gather pipeline (fast arithmetic, packed records)
-        launch(s.early, k_force_tma<3>, s.grid_p, s.tile + 32, force_tma_smem(s.tile), st, a, *static_cast<const CUtensorMap*>(s.fmap));
+        k_force_tma<3><<<s.grid_p, s.tile + 32, force_tma_smem(s.tile), st>>>(a, *static_cast<const CUtensorMap*>(s.fmap));
         return;
     }
     if (s.variant & 8) {
         const bool fast = (s.variant & (131072 | 16)) == (131072 | 16);
         if (!s.pack) {
             if (fast)
-                launch(s.early, k_force<false, 4, true, true, true>, s.grid_dyn, s.tile, 0, st, a);
+                k_force<false, 4, true, true, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
             else
-                launch(s.early, k_force<false, 4, true, true>, s.grid_dyn, s.tile, 0, st, a);
+                k_force<false, 4, true, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
         } else if (s.record) {
             if (fast)
-                launch(s.early, k_force_rec<true, true>, s.grid_dyn, s.tile, 0, st, a);
+                k_force_rec<true, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
             else
-                launch(s.early, k_force_rec<false, true>, s.grid_dyn, s.tile, 0, st, a);
+                k_force_rec<false, true><<<s.grid_dyn, s.tile, 0, st>>>(a);
         } else if (fast)
-            launch(s.early, k_force_rec<true, false>, s.grid_dyn, s.tile, 0, st, a);
+            k_force_rec<true, false><<<s.grid_dyn, s.tile, 0, st>>>(a);
         else
-            launch(s.early, k_force_rec<false, false>, s.grid_dyn, s.tile, 0, st, a);
+            k_force_rec<false, false><<<s.grid_dyn, s.tile, 0, st>>>(a);
     } else if (s.variant & 4)
-        launch(s.early, k_force<false, 3>, s.grid_p, s.tile, list_bytes(s), st, a);
+        k_force<false, 3><<<s.grid_p, s.tile, list_bytes(s), st>>>(a);
     else
-        launch(s.early, k_force<false, 4>, s.grid_p, s.tile, list_bytes(s), st, a);
+        k_force<false, 4><<<s.grid_p, s.tile, list_bytes(s), st>>>(a);
 }
 void launch_force_ordered(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     if (s.ordered_group)
         launch(s.early, k_force_ordered, s.grid_p * s.tile / 8, 256, 0, st, a);
     else
-        launch(s.early, k_force<true, 1>, s.grid_p, s.tile, 0, st, a);
+        k_force<true, 1><<<s.grid_p, s.tile, 0, st>>>(a);
 }
 void launch_terrain(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     launch(s.early, k_terrain, (s.grid_t * (s.tile / 4) + 255) / 256, 256, 0, st, a);
