@@ -1513,12 +1513,16 @@ __global__ void __launch_bounds__(kMaxTile, FM ? 3 : 4) k_force_rec(const __grid
             const PairConst K = {S.h, S.hh, FM ? 3.0f * S.hh : fm(fm(3.0f, S.h), S.h), S.c_grad, S.c_spiky, S.mass,
                                  FM ? S.cthr * S.cthr : S.cthr, neg_zero()};
             // pairs closer than the threshold (with a margin) take the general
-            // form, and so do all pairs of a particle whose own velocity or
-            // factors are not finite (zero times those is not zero)
+            // form, and so do all pairs of a particle whose own velocity, or a
+            // factor of its pair with itself, is not finite (zero times those
+            // is not zero)
             const Rec me = ld_rec(fd + 2 * pl);
             const float nxi = -lo(me.xy), nyi = -hi(me.xy), nzi = -lo(me.zA), Ai = hi(me.zA);
             const float nvx = -lo(me.vxy), nvy = -hi(me.vxy), nvz = -lo(me.vzB);
-            const bool odd = !((nvx + nvy + nvz) * 0.0f + (Ai + hi(me.vzB)) * 0.0f == 0.0f);
+            const float coef = (Ai + Ai) * K.mass;
+            const float own = (FM ? coef * K.cs * (K.h * K.h) * rsqrtf(K.clamp) : coef) +
+                              hi(me.vzB) * (K.h * K.cs) + hi(me.vzB) * K.cg * (K.hh * K.hh) + K.hh * K.cg * K.hh3;
+            const bool odd = !((nvx + nvy + nvz) * 0.0f + own * 0.0f == 0.0f);
             const float c2 = odd ? INFINITY : S.cthr * S.cthr * 1.0001f;
             const bool rec = REC && (S.flags & kFlagRecord) != 0;
             // the list, two entries at a time; past its end: the particle itself
