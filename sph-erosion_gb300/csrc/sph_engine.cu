@@ -320,17 +320,33 @@ int64_t System::scene_bytes(int n, int tw, int td, const sph_params& p, bool lis
            round_up((int64_t)tw * td, kTAlign) * 16 + (int64_t)(pcap / cfg_.tile + tmp.nchunks) * 8;
 }
 
-void System::check_budget(int64_t extra) {
-    if (cfg_.hbm_budget <= 0 || memory_bytes() + extra <= cfg_.hbm_budget) return;
-    // packed records that the variant does not ask for make way
-    if (fdat_.n && !(cfg_.variant & 128)) {
-        SPH_CK(cudaStreamSynchronize(st_));
-        fdat_.release();
-        work_dirty_ = true;
-        drop_graph();
-        if (memory_bytes() + extra <= cfg_.hbm_budget) return;
+// Packed records that the variant does not ask for (ensure_nlist) make way
+// for whatever else needs their memory.  They hold nothing between steps, and
+// the next step takes them again if they still fit.
+bool System::release_optional() {
+    if (!fdat_.n || (cfg_.variant & 128)) return false;
+    SPH_CK(cudaStreamSynchronize(st_));
+    fdat_.release();
+    work_dirty_ = true;
+    drop_graph();
+    return true;
+}
+
+template <class T>
+void System::resize(DevBuf<T>& b, int64_t cnt, bool keep) {
+    try {
+        b.resize(cnt, keep, st_);
+    } catch (const Error& e) {
+        if (e.code != SPH_ERR_NOMEM) throw;
+        cudaGetLastError();
+        if (!release_optional()) throw;
+        b.resize(cnt, keep, st_);
     }
-    throw Error(SPH_ERR_CAPACITY, "HBM budget exceeded");
+}
+
+void System::check_budget(int64_t extra) {
+    auto over = [&] { return cfg_.hbm_budget > 0 && memory_bytes() + extra > cfg_.hbm_budget; };
+    if (over() && !(release_optional() && !over())) throw Error(SPH_ERR_CAPACITY, "HBM budget exceeded");
 }
 
 void System::drop_graph() {
@@ -346,13 +362,13 @@ void System::grow_particles(int64_t cap) {
     if (need <= 0) return;
     check_budget(need * (5 * 16 + 3 * 4 + 2 * 4 + (rec_.n ? kRecFloats * 4 : 0)));
     DevBuf<float4>* f4[] = {&pos_, &vel_, &spos_, &svel_, &dyn_};
-    for (auto* b : f4) b->resize(cap, true, st_);
-    key_.resize(cap, true, st_);
-    slot_.resize(cap, true, st_);
-    perm_.resize(cap, true, st_);
-    nbid_.resize(cap, true, st_);
-    snbid_.resize(cap, true, st_);
-    if (rec_.n) rec_.resize(cap * kRecFloats, true, st_);
+    for (auto* b : f4) resize(*b, cap, true);
+    resize(key_, cap, true);
+    resize(slot_, cap, true);
+    resize(perm_, cap, true);
+    resize(nbid_, cap, true);
+    resize(snbid_, cap, true);
+    if (rec_.n) resize(rec_, cap * kRecFloats, true);
     pa_.grow(cap);
     work_dirty_ = true;  // the neighbour lists follow the arena's size
     drop_graph();
@@ -360,29 +376,29 @@ void System::grow_particles(int64_t cap) {
 void System::grow_keys(int64_t cap) {
     if (cap <= counts_.n) return;
     check_budget((cap - counts_.n) * 8);
-    counts_.resize(cap, true, st_);
-    offsets_.resize(cap, true, st_);
+    resize(counts_, cap, true);
+    resize(offsets_, cap, true);
     ka_.grow(cap);
     drop_graph();
 }
 void System::grow_chunks(int64_t cap) {
     if (cap <= chunk_.n) return;
-    chunk_.resize(cap, true, st_);
+    resize(chunk_, cap, true);
     ca_.grow(cap);
     drop_graph();
 }
 void System::grow_tables(int64_t cap) {
     if (cap <= tab_.n) return;
-    tab_.resize(cap, true, st_);
+    resize(tab_, cap, true);
     tba_.grow(cap);
     drop_graph();
 }
 void System::grow_terrain(int64_t cap) {
     if (cap <= tbase_.n) return;
     check_budget((cap - tbase_.n) * 16);
-    tbase_.resize(cap, true, st_);
-    theight_.resize(cap, true, st_);
-    tdelta_.resize(cap, true, st_);
+    resize(tbase_, cap, true);
+    resize(theight_, cap, true);
+    resize(tdelta_, cap, true);
     ta_.grow(cap);
     drop_graph();
 }
@@ -617,7 +633,7 @@ int System::create_scene(const sph_params& p, int capacity, int tw, int td) {
         }
     }
     if (p.flags & SPH_FLAG_RECORD && rec_.n == 0) {
-        rec_.resize(pos_.n * kRecFloats, false, st_);
+        resize(rec_, pos_.n * kRecFloats, false);
         drop_graph();
     }
     // row tables and clean key ranges
@@ -709,7 +725,7 @@ void System::set_params(int id, const sph_params& p) {
     }
     if ((p.flags & SPH_FLAG_RECORD) && rec_.n == 0) {
         SPH_CK(cudaStreamSynchronize(st_));
-        rec_.resize(pos_.n * kRecFloats, false, st_);
+        resize(rec_, pos_.n * kRecFloats, false);
         drop_graph();
     }
     if ((p.flags ^ sc.prm.flags) & (SPH_FLAG_ORDERED | SPH_FLAG_RECORD)) work_dirty_ = true;
@@ -811,7 +827,7 @@ void System::get_particles(int id, float* pos3, float* vel3, float* density, int
     const int n = sc.n;
     if (n == 0) return;
     // gather into id order on the device, then copy only what was asked for
-    if (stage_.n < (int64_t)8 * n) stage_.resize((int64_t)8 * n, false, st_);
+    if (stage_.n < (int64_t)8 * n) resize(stage_, (int64_t)8 * n, false);
     float* d_pos = stage_.p;
     float* d_vel = stage_.p + (size_t)3 * n;
     float* d_den = stage_.p + (size_t)6 * n;
@@ -843,7 +859,7 @@ void System::get_particles_async(int id, float* pos3, float* vel3, float* densit
     aslot_ ^= 1;
     if (astage_[k].n < (int64_t)8 * n) {
         SPH_CK(cudaStreamSynchronize(cst_));
-        astage_[k].resize((int64_t)8 * n, false, st_);
+        resize(astage_[k], (int64_t)8 * n, false);
     }
     SPH_CK(cudaStreamWaitEvent(st_, copied_[k], 0));
     float* d_pos = astage_[k].p;
@@ -911,9 +927,9 @@ void System::diag_many(const int* ids, int k, sph_diag* out) {
     for (int q = 0; q < k; ++q) scene(ids[q]);
     if (work_dirty_) rebuild_work();
     if (diag_part_.n < (int64_t)k * kDiagBlocks * kDiagDoubles)
-        diag_part_.resize((int64_t)k * kDiagBlocks * kDiagDoubles, false, st_);
-    if (diag_i_.n < (int64_t)3 * k) diag_i_.resize((int64_t)3 * k, false, st_);
-    if (diag_nan_.n < k) diag_nan_.resize(k, false, st_);
+        resize(diag_part_, (int64_t)k * kDiagBlocks * kDiagDoubles, false);
+    if (diag_i_.n < (int64_t)3 * k) resize(diag_i_, (int64_t)3 * k, false);
+    if (diag_nan_.n < k) resize(diag_nan_, k, false);
     SPH_CK(cudaMemcpyAsync(slist_.p, ids, (size_t)k * sizeof(int), cudaMemcpyHostToDevice, st_));
     SPH_CK(cudaMemsetAsync(diag_i_.p, 0, (size_t)3 * k * sizeof(long long), st_));
     SPH_CK(cudaMemsetAsync(diag_nan_.p, 0, (size_t)k * sizeof(int), st_));
@@ -1045,7 +1061,7 @@ void System::rebuild_work() {
         if (sc.live && sc.steps >= 0) any_limited_ = true;
     auto up = [&](DevBuf<Work>& b, const std::vector<Work>& v) {
         if ((int64_t)v.size() > b.n) {
-            b.resize(std::max<int64_t>((int64_t)v.size(), b.n * 2), false, st_);
+            resize(b, std::max<int64_t>((int64_t)v.size(), b.n * 2), false);
             drop_graph();
         }
         if (!v.empty())
@@ -1092,14 +1108,15 @@ void System::ensure_nlist() {
     };
     if (nlist_.n != slots || ncnt_.n != pos_.n || (fdat_.n != need && fdat_.n != want)) {
         if (!fits(need)) return;
-        nlist_.resize(slots, false, st_);
-        ncnt_.resize(pos_.n, false, st_);
+        fdat_.release();  // holds nothing between steps: first, so that the lists have its room
+        resize(nlist_, slots, false);
+        resize(ncnt_, pos_.n, false);
         drop_graph();
     }
     if (fdat_.n != want) {
         int64_t recs = fits(want) ? want : need;
         if (fdat_.n != recs) {
-            fdat_.release();  // holds nothing between steps
+            fdat_.release();
             if (recs) try {
                     fdat_.resize(recs, false, st_);
                 } catch (const Error& e) {
@@ -1407,7 +1424,7 @@ void System::traversal_stats(int id, int64_t* out4) {
     if (sc.n == 0) return;
     const DevArrays a = arrays();
     enqueue_sort(a, shape());
-    if (diag_i_.n < 4) diag_i_.resize(4, false, st_);
+    if (diag_i_.n < 4) resize(diag_i_, 4, false);
     SPH_CK(cudaMemsetAsync(diag_i_.p, 0, 4 * sizeof(long long), st_));
     launch_traversal_stats(a, id, reinterpret_cast<unsigned long long*>(diag_i_.p), st_);
     SPH_CK(cudaGetLastError());
@@ -1423,7 +1440,7 @@ void System::neighbour_counts(int id, int32_t* out) {
     Scene& sc = scene(id);
     if (work_dirty_) rebuild_work();
     if (sc.n == 0) return;
-    if (scratch_i_.n < pos_.n) scratch_i_.resize(pos_.n, false, st_);
+    if (scratch_i_.n < pos_.n) resize(scratch_i_, pos_.n, false);
     const DevArrays a = arrays();
     enqueue_sort(a, shape());
     launch_neighbour_counts(a, shape(), scratch_i_.p, st_);
@@ -1446,11 +1463,11 @@ void System::autotune(int steps, sph_tune_result* out) {
     DevBuf<int32_t> snb;
     DevBuf<long long> sdel;
     DevBuf<float> shgt;
-    spos.resize(np, false, st_);
-    svel.resize(np, false, st_);
-    snb.resize(np, false, st_);
-    sdel.resize(nt, false, st_);
-    shgt.resize(nt, false, st_);
+    resize(spos, np, false);
+    resize(svel, np, false);
+    resize(snb, np, false);
+    resize(sdel, nt, false);
+    resize(shgt, nt, false);
     auto copy = [&](void* dst, const void* src, size_t bytes) {
         if (bytes) SPH_CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, st_));
     };

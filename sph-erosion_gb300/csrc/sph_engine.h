@@ -116,6 +116,7 @@ class System {
 
     void step(int nsteps);
     void sync();
+    bool release_optional();  // gives back the packed records that are held only for speed; false: none
     bool trim();  // with no live scene: back to the initial arena sizes
     void autotune(int steps, sph_tune_result* out);
     float time_steps(int nsteps);
@@ -156,6 +157,10 @@ class System {
     void advance_step_mirror(int nsteps);
     void drop_graph();
     void check_budget(int64_t extra);
+    // DevBuf::resize; without device memory for it, again once the optional
+    // buffers are given back
+    template <class T>
+    void resize(DevBuf<T>& b, int64_t cnt, bool keep);
     void upload_terrain_height(Scene& sc);
 
     sph_system_config cfg_;

@@ -111,11 +111,18 @@ __global__ void k_mesh_f32(const float* __restrict__ h, int tw, int td, float xl
     o[5] = n.z;
 }
 
-// Temporary device buffers of one mesh call.
+// Temporary device buffers of one mesh call.  Without memory for one, the
+// system whose terrain it is gives back what it holds only for speed.
 struct Tmp {
     void* p = nullptr;
-    explicit Tmp(size_t bytes) {
-        if (bytes) check_cuda(cudaMalloc(&p, bytes), "cudaMalloc(mesh)");
+    explicit Tmp(size_t bytes, System* sys = nullptr) {
+        if (!bytes) return;
+        cudaError_t e = cudaMalloc(&p, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            if (sys && sys->release_optional()) e = cudaMalloc(&p, bytes);
+        }
+        check_cuda(e, "cudaMalloc(mesh)");
     }
     ~Tmp() {
         if (p) cudaFree(p);
@@ -160,7 +167,7 @@ void mesh_scene(System& sys, int scene, float* verts, unsigned* idx, float metre
     const int64_t nv = (int64_t)tw * td, ni = (int64_t)6 * (tw - 1) * (td - 1);
     std::vector<float> h((size_t)nv);
     sys.get_terrain(scene, h.data(), nullptr);
-    Tmp dh((size_t)nv * 4), dv((size_t)nv * 24), di((size_t)ni * 4);
+    Tmp dh((size_t)nv * 4, &sys), dv((size_t)nv * 24, &sys), di((size_t)ni * 4, &sys);
     check_cuda(cudaMemcpy(dh.p, h.data(), (size_t)nv * 4, cudaMemcpyHostToDevice), "copy heights");
     k_mesh_f32<<<(unsigned)((nv + 255) / 256), 256>>>(static_cast<float*>(dh.p), tw, td, xlo, ylo, zlo, sx, sz, ys,
                                                       static_cast<float*>(dv.p));
