@@ -1513,27 +1513,41 @@ void System::autotune(int steps, sph_tune_result* out) {
     };
     const int tiles[2] = {128, 256};
     const float cms[2] = {1.0f, 0.5f};
-    // per-lane passes (0, 4: cells; 28, 88, 120, 216: lists; 32856, 32888:
-    // the force pass in dynamically scheduled warp slices; 163928, 163960,
-    // 164088: the same in fast arithmetic, 164088 with packed records) and
-    // cooperative passes (264: 32 + 8 lanes per particle, 776: 4 force
-    // lanes, 2312: 16 density lanes).  The TMA gather pipeline (bit 18) is
-    // left out: 3-4x slower than 164088 on every state measured.
+    // per-lane passes (0, 4: cells; 28, 88, 120, 216, 32856, 32888: lists;
+    // 163928, 163960, 164088: the same in fast arithmetic) and cooperative
+    // passes (264: 32 + 8 lanes per particle, 776: 4 force lanes, 2312: 16
+    // density lanes).  The list variants of one arithmetic launch the same
+    // kernels since they share one list walk: such a set is timed once and its
+    // first member, which asks for no more memory than the others, is the one
+    // picked.  The TMA gather pipeline (bit 18) is left out: 3-4x slower than
+    // 163928 on every state measured.
     const int variants[] = {0,      4,      28,     88,  120, 216, 32856, 32888,
                             163928, 163960, 164088, 264, 776, 2312};
     static_assert(2 * 2 * (sizeof variants / sizeof variants[0]) <= 64, "sph_tune_result holds 64 trials");
+    std::vector<std::pair<int, float>> timed[2];  // neighbour kernels and their time, of each tile at one cell size
     float best = 1e30f;
     int bt = cfg_.tile, bv = cfg_.variant;
     float bc = scenes_.empty() ? 1.0f : scenes_[0].prm.cell_mult;
     try {
-        for (float cm : cms)
+        for (float cm : cms) {
+            for (auto& t : timed) t.clear();
             for (int variant : variants)
                 for (int tile : tiles) {
                     apply(tile, cm, variant);
-                    step(2);  // warm-up: graphs captured, caches primed
-                    SPH_CK(cudaStreamSynchronize(st_));
-                    const float ms = time_steps(steps) / (float)steps;
-                    restore();
+                    if (work_dirty_) rebuild_work();
+                    const int kernels = neighbour_kernels(shape());
+                    auto& seen = timed[tile != tiles[0]];
+                    auto same = std::find_if(seen.begin(), seen.end(), [&](auto& t) { return t.first == kernels; });
+                    float ms;
+                    if (same != seen.end()) {
+                        ms = same->second;
+                    } else {
+                        step(2);  // warm-up: graphs captured, caches primed
+                        SPH_CK(cudaStreamSynchronize(st_));
+                        ms = time_steps(steps) / (float)steps;
+                        restore();
+                        seen.push_back({kernels, ms});
+                    }
                     const int k = out->n_tried++;
                     out->tiles[k] = tile;
                     out->cell_mults[k] = cm;
@@ -1546,6 +1560,7 @@ void System::autotune(int steps, sph_tune_result* out) {
                         bv = variant;
                     }
                 }
+        }
         apply(bt, bc, bv);
         restore();
     } catch (...) {

@@ -2893,6 +2893,14 @@ void group_rules(LaunchShape& s) {
 
 static bool coop(const LaunchShape& s) { return (s.variant & (256 | 8)) == (256 | 8); }
 
+// The bits that the launchers below act on, by the form that they take.
+int neighbour_kernels(const LaunchShape& s) {
+    if (coop(s)) return s.variant;
+    if (!(s.variant & 8)) return s.variant & (1 | 4);
+    const bool tma = s.fmap && (s.variant & 128) && !s.force_group;
+    return (s.variant & (8 | 16 | 131072 | (tma ? 262144 : 0))) | (s.pack ? 128 : 0);
+}
+
 void launch_density(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     if (coop(s)) {
         launch_density_coop(a, s, st);

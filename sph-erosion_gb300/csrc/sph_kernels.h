@@ -98,6 +98,8 @@ void launch_keys(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_scan(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_scatter(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_reorder(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
+// Variants with the same value launch the same neighbour kernels.
+int neighbour_kernels(const LaunchShape& s);
 // Sets early and the three group members from the others.
 void group_rules(LaunchShape& s);
 void launch_density(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
