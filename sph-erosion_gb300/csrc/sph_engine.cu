@@ -189,6 +189,7 @@ System::System(const sph_system_config& cfg) : cfg_(cfg) {
     dev_ = cfg_.device;
     SPH_CK(cudaSetDevice(dev_));
     SPH_CK(cudaDeviceGetAttribute(&nsm_, cudaDevAttrMultiProcessorCount, dev_));
+    SPH_CK(cudaDeviceGetStreamPriorityRange(nullptr, &priority_));
     SPH_CK(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
     SPH_CK(cudaStreamCreateWithFlags(&cst_, cudaStreamNonBlocking));
     for (int k = 0; k < 2; ++k) {
@@ -833,7 +834,7 @@ void System::get_particles(int id, float* pos3, float* vel3, float* density, int
     float* d_den = stage_.p + (size_t)6 * n;
     int32_t* d_sed = reinterpret_cast<int32_t*>(stage_.p + (size_t)7 * n);
     launch_gather_by_id(pos_.p, vel_.p, dyn_.p, (int)sc.p_off, n, pos3 ? d_pos : nullptr, vel3 ? d_vel : nullptr,
-                        density ? d_den : nullptr, sed ? d_sed : nullptr, st_);
+                        density ? d_den : nullptr, sed ? d_sed : nullptr, priority_, st_);
     SPH_CK(cudaGetLastError());
     if (pos3) SPH_CK(cudaMemcpyAsync(pos3, d_pos, (size_t)n * 12, cudaMemcpyDeviceToHost, st_));
     if (vel3) SPH_CK(cudaMemcpyAsync(vel3, d_vel, (size_t)n * 12, cudaMemcpyDeviceToHost, st_));
@@ -867,7 +868,7 @@ void System::get_particles_async(int id, float* pos3, float* vel3, float* densit
     float* d_den = astage_[k].p + (size_t)6 * n;
     int32_t* d_sed = reinterpret_cast<int32_t*>(astage_[k].p + (size_t)7 * n);
     launch_gather_by_id(pos_.p, vel_.p, dyn_.p, (int)sc.p_off, n, pos3 ? d_pos : nullptr, vel3 ? d_vel : nullptr,
-                        density ? d_den : nullptr, sed ? d_sed : nullptr, st_);
+                        density ? d_den : nullptr, sed ? d_sed : nullptr, priority_, st_);
     SPH_CK(cudaGetLastError());
     SPH_CK(cudaEventRecord(gathered_[k], st_));
     SPH_CK(cudaStreamWaitEvent(cst_, gathered_[k], 0));

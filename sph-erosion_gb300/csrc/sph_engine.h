@@ -179,6 +179,7 @@ class System {
     DevBuf<float> astage_[2];
     int aslot_ = 0;
     int dev_ = 0, nsm_ = 1;
+    int priority_ = 0;  // highest launch priority of the device
     cudaStream_t st_ = nullptr;
     std::vector<Scene> scenes_;
 

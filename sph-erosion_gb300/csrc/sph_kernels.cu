@@ -2772,9 +2772,24 @@ void launch_traversal_stats(const DevArrays& a, int scene, unsigned long long* o
     k_traversal_stats<<<304, 256, 0, st>>>(a, scene, out);
 }
 
+// The readback's gather, one launch per scene, at the highest priority: its few
+// blocks otherwise wait for every block of the neighbour pass that another
+// system's stream has running, scene after scene.  Three systems of 39 scenes
+// (216,000 particles) in turn, a pass of four steps and the readback, us: fast
+// arithmetic 587 -> 508, exact 704 -> 584.
 void launch_gather_by_id(const float4* pos, const float4* vel, const float4* dyn, int p_off, int n, float* pos3,
-                         float* vel3, float* dens, int32_t* sed, cudaStream_t st) {
-    if (n > 0) k_gather_by_id<<<(n + 255) / 256, 256, 0, st>>>(pos, vel, dyn, p_off, n, pos3, vel3, dens, sed);
+                         float* vel3, float* dens, int32_t* sed, int priority, cudaStream_t st) {
+    if (n <= 0) return;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)((n + 255) / 256));
+    c.blockDim = dim3(256);
+    c.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributePriority;
+    at.val.priority = priority;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, k_gather_by_id, pos, vel, dyn, p_off, n, pos3, vel3, dens, sed);
 }
 
 void configure_kernels() {

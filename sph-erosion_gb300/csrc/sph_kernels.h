@@ -115,7 +115,7 @@ void launch_neighbour_counts(const DevArrays& a, const LaunchShape& s, int32_t* 
 void launch_traversal_stats(const DevArrays& a, int scene, unsigned long long* out, cudaStream_t st);
 // Scatter a scene's state into id order: any output may be null.
 void launch_gather_by_id(const float4* pos, const float4* vel, const float4* dyn, int p_off, int n, float* pos3,
-                         float* vel3, float* dens, int32_t* sed, cudaStream_t st);
+                         float* vel3, float* dens, int32_t* sed, int priority, cudaStream_t st);
 // Per-scene FP64 partial sums: kDiagBlocks blocks per listed scene.
 constexpr int kDiagBlocks = 32;
 constexpr int kDiagDoubles = 8;  // mass-weighted momentum xyz, kinetic, potential, (pad)
