@@ -9,7 +9,6 @@ from __future__ import annotations
 import ctypes as C
 import os
 import subprocess
-import unittest
 
 import numpy as np
 
@@ -268,17 +267,13 @@ def time_sample(params, pos, vel, i0, m, nthreads=0):
 
 
 # ---------------------------------------------------------------------------
-class ReferenceAbsent(FileNotFoundError, unittest.SkipTest):
-    """The reference harness was not built here: a test that needs it is skipped."""
-
-
 class Reference:
     """The reference's own FluidSystemSPH, built headless (only where the
     reference sources are present)."""
 
     def __init__(self):
         if not os.path.exists(REF_PATH):
-            raise ReferenceAbsent(REF_PATH)
+            raise FileNotFoundError(REF_PATH)
         L = C.CDLL(REF_PATH)
         f32p = np.ctypeslib.ndpointer(np.float32, flags="C")
         i32p = np.ctypeslib.ndpointer(np.int32, flags="C")

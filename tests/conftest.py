@@ -17,6 +17,15 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (runs the sm_103a kernels)")
 
 
+def pytest_collection_modifyitems(items):
+    """The one test that runs the reference's own code needs its sources: an
+    empty reference directory counts as none."""
+    if not os.path.isfile("/root/reference/Erosion/fluid_system.h"):
+        for item in items:
+            if item.name == "test_reference_harness_matches_when_present":
+                item.add_marker(pytest.mark.skip(reason="reference sources absent"))
+
+
 @pytest.fixture(scope="session")
 def golden():
     cache = {}
