@@ -1217,6 +1217,8 @@ DevArrays System::arrays() const {
 LaunchShape System::shape() const {
     LaunchShape s;
     s.tile = cfg_.tile;
+    s.captured = false;
+    s.nsm = nsm_;
     s.grid_p = n_ptiles_;
     s.grid_c = n_ctiles_;
     s.grid_t = n_ttiles_;
@@ -1290,7 +1292,8 @@ void System::capture_graph() {
     Range r("sph/capture_graph");
     drop_graph();
     const DevArrays a = arrays();
-    const LaunchShape s = shape();
+    LaunchShape s = shape();
+    s.captured = true;
     SPH_CK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
     for (int i = 0; i < cfg_.graph_steps; ++i) enqueue_step(a, s, nullptr);
     cudaGraph_t g = nullptr;

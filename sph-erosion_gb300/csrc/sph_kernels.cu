@@ -2651,8 +2651,8 @@ __global__ void __launch_bounds__(256) k_diag(DevArrays a, double* partial, long
 
 // Launch of a kernel of the step (step_enter); early: with programmatic
 // serialization.  It hides a kernel's launch behind the one before it: of
-// 18,432 particles or less a step takes 12 us less launched by itself and 1 to
-// 3 in a graph.  In large systems blocks that wait cost more than that (a step,
+// 18,432 particles or less a step takes about 9 us less launched by itself (4
+// steps of 1,000 124 vs 87 us) and 1 to 2 in a graph (64 steps 1,385 vs 1,275).  In large systems blocks that wait cost more than that (a step,
 // us, with and without: 100,000 particles 127 vs 113, 1,048,576 862 vs 818,
 // 8.4M 5,367 vs 4,949): the list passes keep the L1 split of the kernel they
 // overlapped.
@@ -2863,11 +2863,18 @@ static void launch_force_coop(const DevArrays& a, const LaunchShape& s, cudaStre
 
 static void launch_density_group(const DevArrays& a, const LaunchShape& s, bool fast, cudaStream_t st) {
     const int blocks = s.grid_p * s.tile / 8;
+    // Blocks that wait for the one-block sort, the longest kernel of a small
+    // step, hold most of the chip when they are more than two an SM, and other
+    // systems' kernels out of it.  Three systems in turn, 64 captured steps, us,
+    // early or not: 4,096 particles 855 vs 701, 2,500 604 vs 585, 1,500 527 vs
+    // 526; one alone: 1,684 vs 1,683, 1,478 vs 1,486, 1,349 vs 1,380.  Launched
+    // singly it pays at all of these (2,500 particles, 4 steps: 100 vs 112).
+    const bool early = s.early && !(s.captured && s.sort_smem && blocks > 2 * s.nsm);
     const bool lane_lists = !s.force_group, pack = lane_lists && s.pack;
     if (fast)
-        launch(s.early, k_density_group<true>, blocks, 256, 0, st, a, lane_lists, pack);
+        launch(early, k_density_group<true>, blocks, 256, 0, st, a, lane_lists, pack);
     else
-        launch(s.early, k_density_group<false>, blocks, 256, 0, st, a, lane_lists, pack);
+        launch(early, k_density_group<false>, blocks, 256, 0, st, a, lane_lists, pack);
 }
 
 static void launch_force_group(const DevArrays& a, const LaunchShape& s, bool fast, cudaStream_t st) {

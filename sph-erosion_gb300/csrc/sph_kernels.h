@@ -81,6 +81,8 @@ struct LaunchShape {
     bool pack;       // the density pass writes packed records, the force pass gathers them
     size_t sort_smem;  // shared memory of the one-block sort; 0: a scene is too large for it
     bool early;      // few particles: each kernel's launch overlaps the kernel before it
+    bool captured;   // the launches go into a graph
+    int nsm;         // SMs of the device
     bool density_group, force_group, ordered_group;  // few particles: a group of lanes per particle (group_rules)
     bool record;     // some scene keeps its force records (SPH_FLAG_RECORD)
     int grid_dyn;    // grid of the dynamically scheduled neighbour kernels
