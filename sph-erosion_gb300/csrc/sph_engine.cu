@@ -1060,6 +1060,14 @@ void System::rebuild_work() {
     }
     for (const Scene& sc : scenes_)
         if (sc.live && sc.steps >= 0) any_limited_ = true;
+    // the one-block sort takes the scenes by their first tiles: these go first
+    n_scenes_ = 0;
+    if (sort_small_smem(max_n_, max_keys_)) {
+        const auto rest = std::stable_partition(pt.begin(), pt.end(), [&](const Work& w) {
+            return w.start == (int)scenes_[w.scene].p_off;
+        });
+        n_scenes_ = (int)(rest - pt.begin());
+    }
     auto up = [&](DevBuf<Work>& b, const std::vector<Work>& v) {
         if ((int64_t)v.size() > b.n) {
             resize(b, std::max<int64_t>((int64_t)v.size(), b.n * 2), false);
@@ -1225,6 +1233,7 @@ LaunchShape System::shape() const {
     s.variant = nl_ready_ ? cfg_.variant : (cfg_.variant & ~504);
     s.record = any_record_;
     s.sort_smem = sort_small_smem(max_n_, max_keys_);
+    s.grid_sort = n_scenes_;
     group_rules(s);
     s.pack = nl_ready_ && fdat_.n > 0;
     // enough blocks to fill every SM (2048 threads each); blocks that start

@@ -220,6 +220,7 @@ class System {
     DevBuf<long long> diag_i_;
     DevBuf<int> diag_nan_;
 
+    int n_scenes_ = 0;  // of the one-block sort
     int n_ptiles_ = 0, n_ctiles_ = 0, n_ttiles_ = 0;
     bool any_fast_ = false, any_ordered_ = false, any_terrain_ = false, any_limited_ = false,
          any_record_ = false;

@@ -772,7 +772,8 @@ __global__ void __launch_bounds__(kMaxTile) k_reorder(DevArrays a) {
 // The whole sort of a small scene in one block: keys, scan, scatter and reorder
 // with the counts, offsets and order in shared memory.  The four kernels are
 // chains of dependent loads of 5 to 9 us each at these sizes, whatever the
-// number of particles.  Block w takes the scene whose first tile work item w is.
+// number of particles.  The work list of a system that takes this sort begins with
+// the scenes' first tiles: block w takes the scene of item w.
 constexpr int kSortThreads = 1024;
 constexpr int kSortPer = kSmallSort / kSortThreads;  // particles a thread takes
 
@@ -784,7 +785,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_small(const __grid_consta
     if (a.ctr && blockIdx.x == 0 && tid < 2) a.ctr[tid] = 0u;  // for this step's neighbour kernels
     const Work wk = a.ptiles[blockIdx.x];
     const SceneDev& S = a.scenes[wk.scene];
-    if (wk.start != S.p_off || a.steps_left[wk.scene] == 0) return;
+    if (a.steps_left[wk.scene] == 0) return;
     const int n = S.n, nkeys = S.nkeys;
     const int per = ((nkeys + kSortThreads - 1) / kSortThreads) | 1;  // keys a thread scans; odd: no bank conflicts
     uint32_t* perm = sm;                 // kSmallSort
@@ -2686,7 +2687,7 @@ void launch(bool early, void (*k)(P...), int grid, int block, size_t smem, cudaS
 }  // namespace
 
 void launch_sort_small(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
-    launch(s.early, k_sort_small, s.grid_p, kSortThreads, s.sort_smem, st, a);
+    launch(s.early, k_sort_small, s.grid_sort, kSortThreads, s.sort_smem, st, a);
 }
 size_t sort_small_smem(int64_t max_n, int64_t max_keys) {
     const int64_t per = ((max_keys + kSortThreads - 1) / kSortThreads) | 1;

@@ -80,6 +80,7 @@ struct LaunchShape {
     int variant;     // sph_system_config.variant bits (bit 3 only with lists allocated)
     bool pack;       // the density pass writes packed records, the force pass gathers them
     size_t sort_smem;  // shared memory of the one-block sort; 0: a scene is too large for it
+    int grid_sort;     // its blocks: one per scene, whose first tiles lead the work list
     bool early;      // few particles: each kernel's launch overlaps the kernel before it
     bool captured;   // the launches go into a graph
     int nsm;         // SMs of the device
