@@ -1041,12 +1041,14 @@ void System::rebuild_work() {
     std::vector<Work> pt, ct, tt;
     any_fast_ = any_ordered_ = any_terrain_ = any_limited_ = any_record_ = false;
     max_n_ = max_keys_ = 0;
+    crowded_ = false;
     const int tile = cfg_.tile;
     for (int id = 0; id < (int)scenes_.size(); ++id) {
         const Scene& sc = scenes_[id];
         if (!sc.live || sc.n == 0) continue;
         max_n_ = std::max<int64_t>(max_n_, sc.n);
         max_keys_ = std::max<int64_t>(max_keys_, sc.k_cap);
+        crowded_ |= sort_crowded(sc.n, sc.nkeys);
         for (int t = 0; t * tile < sc.n; ++t) pt.push_back({id, (int)sc.p_off + t * tile});
         for (int c = 0; c < sc.nchunks; ++c) ct.push_back({id, c});
         if (sc.tw > 0)
@@ -1062,7 +1064,7 @@ void System::rebuild_work() {
         if (sc.live && sc.steps >= 0) any_limited_ = true;
     // the one-block sort takes the scenes by their first tiles: these go first
     n_scenes_ = 0;
-    if (sort_small_smem(max_n_, max_keys_)) {
+    if (!crowded_ && sort_small_smem(max_n_, max_keys_)) {
         const auto rest = std::stable_partition(pt.begin(), pt.end(), [&](const Work& w) {
             return w.start == (int)scenes_[w.scene].p_off;
         });
@@ -1232,7 +1234,7 @@ LaunchShape System::shape() const {
     s.grid_t = n_ttiles_;
     s.variant = nl_ready_ ? cfg_.variant : (cfg_.variant & ~504);
     s.record = any_record_;
-    s.sort_smem = sort_small_smem(max_n_, max_keys_);
+    s.sort_smem = crowded_ ? 0 : sort_small_smem(max_n_, max_keys_);
     s.grid_sort = n_scenes_;
     group_rules(s);
     s.pack = nl_ready_ && fdat_.n > 0;

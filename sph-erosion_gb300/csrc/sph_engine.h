@@ -225,6 +225,7 @@ class System {
     bool any_fast_ = false, any_ordered_ = false, any_terrain_ = false, any_limited_ = false,
          any_record_ = false;
     int64_t max_n_ = 0, max_keys_ = 0;  // largest scene of the work lists
+    bool crowded_ = false;              // one of them has too full cells for the one-block sort
     bool work_dirty_ = true;
 
     cudaGraph_t graph_ = nullptr;

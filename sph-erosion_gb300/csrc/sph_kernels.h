@@ -96,6 +96,12 @@ void configure_kernels();
 // Shared memory of the one-block sort for scenes of at most max_n particles and
 // max_keys keys; 0: too large for it.
 size_t sort_small_smem(int64_t max_n, int64_t max_keys);
+// Its block ranks a cell's particles against one another by itself, so a scene
+// of more than two particles a thread whose average cell holds more than 16
+// (cells of 4h and more) is not for it.  4,096 particles, 64 steps, us, one block
+// and the whole chip: cells of 8h 6,821 vs 4,713, of 4h 3,113 vs 2,638 (three
+// systems in turn 1,313 vs 1,388); 2,000 particles, cells of 4h 2,103 vs 2,247.
+constexpr bool sort_crowded(int64_t n, int64_t keys) { return n > 2048 && n > 16 * keys; }
 void launch_sort_small(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_keys(const DevArrays& a, const LaunchShape& s, cudaStream_t st);
 void launch_scan(const DevArrays& a, const LaunchShape& s, cudaStream_t st);

@@ -196,7 +196,7 @@ extern "C" SPH_API int sph_density_static(const sph_params* p, int n, const floa
         s.early = true;
         s.captured = false;
         s.nsm = 0;
-        s.sort_smem = sort_small_smem(n, sc.k_cap);
+        s.sort_smem = sort_crowded(n, sc.nkeys) ? 0 : sort_small_smem(n, sc.k_cap);
         s.grid_sort = 1;
         s.ordered_group = false;
         s.density_group = true;  // at most 32,768 particles (group_rules)

@@ -16,7 +16,7 @@ RULE = r"""
 #include "sph_kernels.h"
 int main() {
     long long n, k;
-    while (scanf("%lld %lld", &n, &k) == 2) printf("%zu\n", sph::sort_small_smem(n, k));
+    while (scanf("%lld %lld", &n, &k) == 2) printf("%zu %d\n", sph::sort_small_smem(n, k), sph::sort_crowded(n, k));
 }
 """
 BLOCK = 227 * 1024  # shared memory that a block can have
@@ -24,7 +24,7 @@ BLOCK = 227 * 1024  # shared memory that a block can have
 
 @pytest.fixture(scope="module")
 def rule(tmp_path_factory):
-    """The sort's shared memory for (particles, keys) pairs."""
+    """(shared memory, crowded?) of (particles, keys) pairs."""
     import build
 
     build.build()
@@ -39,7 +39,7 @@ def rule(tmp_path_factory):
     def ask(sizes):
         out = subprocess.run([str(exe)], input="\n".join(f"{n} {k}" for n, k in sizes), capture_output=True, text=True,
                              check=True).stdout.split()
-        return list(map(int, out))
+        return list(zip(map(int, out[::2]), map(int, out[1::2])))
 
     return ask
 
@@ -47,18 +47,24 @@ def rule(tmp_path_factory):
 def test_rule(rule):
     """At most 4,096 particles and 45,056 keys (key ranges are multiples of 4,096)."""
     sizes = list(itertools.product([1, 4095, 4096, 4097], [4096, 8192, 40960, 45056, 49152, 1 << 20]))
-    for (n, k), smem in zip(sizes, rule(sizes)):
+    for (n, k), (smem, _) in zip(sizes, rule(sizes)):
         assert (smem > 0) == (n <= 4096 and k <= 45056), (n, k, smem)
         assert smem == 0 or (4096 + k) * 4 <= smem <= BLOCK - 2048, (n, k, smem)
 
 
-def states(sizes, dims, fill, tile, clump):
+def test_crowded_cells(rule):
+    """More than 16 particles to a key, where a thread has more than two particles."""
+    sizes = [(1, 2), (2048, 2), (2049, 2), (2049, 128), (2049, 129), (4096, 255), (4096, 256)]
+    assert [c for _, c in rule(sizes)] == [0, 0, 1, 1, 0, 1, 0]
+
+
+def states(sizes, dims, fill, tile, clump, cell_mult=0.5):
     """Keys, order and state after three steps of scenes with grids of dims
     cells, the second scene stopped after one, beside `fill` other particles."""
     rng = np.random.default_rng(5)
     cell = REF["smoothing_radius"] * 0.5 * (1 + 2.0 ** -12)  # cells of h/2
     half = np.array(dims) * (cell / 2) * 0.9999
-    prm = dict(REF, cell_mult=0.5, box_half=tuple(half), dt=1e-3)
+    prm = dict(REF, cell_mult=cell_mult, box_half=tuple(half), dt=1e-3)
     out = []
     with S.System(particle_capacity=sum(sizes) + fill, tile=tile) as sysm:
         scenes = []
@@ -91,4 +97,12 @@ CASES.append(([1, 33, 1000, 4096, 2], (35, 33, 39)))
 @pytest.mark.parametrize("sizes,dims", CASES)
 def test_same_order_and_state(sizes, dims, tile, clump):
     for a, b in zip(states(sizes, dims, 0, tile, clump), states(sizes, dims, 5000, tile, clump)):
+        assert np.array_equal(a, b, equal_nan=a.dtype.kind == "f")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2048, 2049, 4096])
+@pytest.mark.parametrize("cell_mult", [1.0, 4.0, 8.0])
+def test_full_cells(n, cell_mult):
+    for a, b in zip(states([n], (16, 16, 16), 0, 256, 0.0, cell_mult), states([n], (16, 16, 16), 5000, 256, 0.0, cell_mult)):
         assert np.array_equal(a, b, equal_nan=a.dtype.kind == "f")
