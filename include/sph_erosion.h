@@ -169,8 +169,8 @@ SPH_API int sph_system_sync(sph_system* s);  /* waits for steps and asynchronous
 SPH_API int sph_system_time_steps(sph_system* s, int nsteps, float* ms);
 /* Device time per stage of one step, averaged over nsteps (stages: keys, scan,
  * scatter, reorder, density, force, terrain, tick); ms must hold 8 floats.
- * Small scenes (4,096 particles, about 49,000 grid keys) are sorted by one
- * kernel, timed under keys. */
+ * Where every scene is small (4,096 particles, 45,056 grid keys) one kernel
+ * sorts them, timed under keys. */
 SPH_API int sph_system_profile_stages(sph_system* s, int nsteps, float* ms);
 /* Bytes of device memory the system holds. */
 SPH_API int sph_system_memory(sph_system* s, int64_t* bytes);

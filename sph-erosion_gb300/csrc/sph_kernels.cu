@@ -1,12 +1,14 @@
 // Hand-written sm_103a kernels of one simulation step, all scenes of a system
-// per launch.  Each kernel walks a work list of (scene, tile) items in a
-// grid-stride loop; the particle passes are launched with one block per tile,
-// so the hardware hands tiles to SMs as they free up.  A scene whose step
-// budget is exhausted is skipped.
+// per launch.  Work is a list of (scene, tile) items: a block per tile, which
+// the hardware hands to SMs as they free up; warps that take slices of tiles
+// from a counter (the force pass over lists); or, in small systems, a group of
+// lanes per particle of a tile.  A scene whose step budget is exhausted is
+// skipped.
 //
 // Stage order per step (the reference's Run, Erosion/fluid_system.h:104-183,
 // with its three O(N^2) passes replaced by a uniform grid):
-//   keys -> scan -> scatter -> reorder   counting sort into Morton-ordered cell rows along x
+//   keys -> scan -> scatter -> reorder   counting sort into Morton-ordered cell rows along x;
+//                                         one kernel where every scene is small (sort_small_smem)
 //   density                               pass 1 (:107-124)
 //   force                                 passes 2 and 3 (:127-178), advance
 //                                         (:306-353), box (:355-407), terrain
@@ -1128,9 +1130,10 @@ __device__ __forceinline__ float density_sum_exact(const DevArrays& a, const Sce
 // a square root, sums over the finished list, where every lane of the warp has
 // a pair to evaluate.  No unit bounds it (instructions 65%, L1 data path 60%):
 // the rows are walked in step, which keeps a warp's loads in few cache lines
-// but leaves 40% of the lanes waiting for the longest row.  80 registers: at 64
-// the compiler spills (437 where these take 327 us), 16 warps an SM are too few
-// (392).  1,048,576 particles, before and after: fast, cells of h/2, 380 ->
+// but leaves 40% of the lanes waiting for the longest row.  80 registers: with 64
+// or 72 the loads of four candidates are no longer all in flight (exact, cells
+// of h: 535 and 478 us where these take 435; fast, cells of h/2: 409 and 351,
+// 312), and 16 warps an SM are too few (392).  1,048,576 particles, before and after: fast, cells of h/2, 380 ->
 // 315 us; exact, cells of h, 488 -> 439 us.
 template <bool FM>
 __global__ void __launch_bounds__(kMaxTile, 3) k_density_list(const __grid_constant__ DevArrays a, bool pack) {
@@ -2524,7 +2527,8 @@ size_t force_tma_smem(int tile) {
 // with 16-byte loads and stores (a scene's vertices start on a 512-vertex
 // boundary, so every thread's first vertex is 4-aligned).  A block takes 1024 /
 // T tiles: with one tile, a warp or two, the blocks' own overhead was a third
-// of the time (16.8 million vertices, tile 128: 72 -> 45 us, 7.4 TB/s).
+// of the time (16.8 million vertices, tile 128: 72 -> 45 us, 5.96 TB/s of 16 B a
+// vertex).
 __global__ void __launch_bounds__(256) k_terrain(DevArrays a) {
     step_enter(a.early);
     const int nwork = *a.n_ttiles, T4 = a.tile / 4, per = 256 / T4;
@@ -2807,11 +2811,9 @@ static size_t list_bytes(const LaunchShape& s) { return (size_t)kListCap * s.til
 // Variant bit 2 relaxes the register budget of the two neighbour kernels
 // (fewer resident blocks, no spills) against the default high occupancy.
 // Bit 3 hands the in-range neighbour lists from the density pass to the force
-// pass (takes precedence over bit 0); bit 4 with it pipelines the force
-// pass's list walk; bit 5 with it relaxes the density pass's register
-// budget alone (4 resident blocks of 256 threads); bit 6 pairs the density pass's
-// candidate loads; bit 7 with bit 3 packs each particle's force-pass inputs
-// into one 32-byte record.
+// pass (takes precedence over bit 0) and ignores bit 2; bits 4 and 17 with it
+// select the fast arithmetic of the force pass, bit 17 that of the density pass;
+// bit 7 makes the packed 32-byte records part of the variant's memory.
 // Variant bit 8 (with bit 3): the cooperative passes, G lanes per particle.
 // Density: 32 lanes (bit 11: 16).  Force: 8 lanes (bit 9: 4, bit 10: 16).
 // Bit 7 packs the force-pass inputs as in the per-lane passes; bit 2
@@ -2968,7 +2970,7 @@ void launch_force(const DevArrays& a, const LaunchShape& s, cudaStream_t st) {
     // lane: over the packed records wherever the system holds them, since that
     // form is the fastest at every size measured; warps take their work in
     // slices from a counter.
-    if (!s.force_group && (s.variant & 262144) && (s.variant & (131072 | 128 | 24)) == (131072 | 128 | 24) && s.fmap) {
+    if ((s.variant & 262144) && (s.variant & (131072 | 128 | 24)) == (131072 | 128 | 24) && s.fmap) {
         // bit 18: the TMA gather pipeline (fast arithmetic, packed records)
         k_force_tma<3><<<s.grid_p, s.tile + 32, force_tma_smem(s.tile), st>>>(a, *static_cast<const CUtensorMap*>(s.fmap));
         return;

@@ -68,7 +68,8 @@ struct DevArrays {
 constexpr int kNbCap = 192;
 
 // The one-block sort of small scenes: most particles, and most shared memory
-// (counts for 49,000 keys beside the order).
+// (counts for 45,056 keys beside the order: the scan's odd share of a thread
+// rounds the next key range, 49,152, up to 2 KB more).
 constexpr int kSmallSort = 4096;
 constexpr int kSmallSortBytes = 215040;
 
